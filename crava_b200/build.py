@@ -23,7 +23,16 @@ SOURCES = {
     "capi.cu": [],
     "fft.cu": [],
     "cols_tma.cu": [],
+    "pass.cu": [],
     "plane.cu": [],
+    "fft_len0.cu": [],
+    "fft_len1.cu": [],
+    "fft_len2.cu": [],
+    "fft_len3.cu": [],
+    "fft_len4.cu": [],
+    "fft_len5.cu": [],
+    "fft_len6.cu": [],
+    "fft_len7.cu": [],
     "solve.cu": [],
     "solve_ref.cu": ["-fmad=false"],
     "sim.cu": ["-fmad=false"],

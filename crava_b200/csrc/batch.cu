@@ -71,31 +71,17 @@ bool disjoint(const crava_gpu_ctx *c, const crava_gpu_grids *in, const crava_gpu
 int run_vintage_head(const crava_gpu_batch::Vintage &v) {
   crava_gpu_ctx *c = v.ctx;
   if (v.nsim == 0) return run_unit(c, &v.in, &v.out, v.precision);
-  const int nt = c->p.ntheta;
   const crava_gpu_grids &in = v.in, &out = v.out;
   int rc;
   CRAVA_CUDA_TRY(cudaMemsetAsync(c->counters, 0, sizeof(DevCounters), c->stream));
   if ((rc = stage_event(c, 0))) return rc;
-  for (int q = 0; q < 3; ++q)
-    if ((rc = pass_forward(c, in.mu[q], out.mu[q], CRAVA_GRID_PARAMETER))) return rc;
-  for (int l = 0; l < nt; ++l)
-    if ((rc = pass_forward(c, in.data[l], out.data[l], CRAVA_GRID_DATA))) return rc;
-  // the band-gated covariance rule in the forward z passes (as run_unit)
-  ZPrior zp[6];
   bool gated = false;
-  if ((rc = gated_prior_setup(c, v.precision, zp, &gated))) return rc;
-  for (int t = 0; t < 6; ++t)
-    if ((rc = pass_forward(c, in.cov[t], out.cov[t], CRAVA_GRID_COVARIANCE, gated ? &zp[t] : nullptr))) return rc;
-  if ((rc = pass_forward(c, in.err_corr, out.err_corr, CRAVA_GRID_COVARIANCE))) return rc;
-  if (gated && (rc = gated_prior_count(c))) return rc;
+  if ((rc = unit_forward(c, &in, &out, v.precision, &gated))) return rc;
   if ((rc = stage_event(c, 1))) return rc;
   if ((rc = pass_solve(c, &out, v.precision, gated))) return rc;
   if ((rc = stage_event(c, 2))) return rc;
-  for (int q = 0; q < 3; ++q)
-    if ((rc = pass_inverse(c, out.mu[q], CRAVA_GRID_PARAMETER))) return rc;
-  for (int l = 0; l < nt; ++l)
-    if ((rc = pass_inverse(c, out.data[l], CRAVA_GRID_DATA))) return rc;
-  return CRAVA_GPU_OK;
+  // means and residuals lead the unit's order
+  return unit_inverse(c, &out, 0, 3 + c->p.ntheta);
 }
 
 // The rest of a vintage with realisations, after the batch's realisation
@@ -108,8 +94,7 @@ int run_vintage_tail(const crava_gpu_batch::Vintage &v) {
   int rc;
   const float *pm[3] = {out.mu[0], out.mu[1], out.mu[2]};
   if ((rc = inverse_realisations(c, v.sim.data(), 3 * v.nsim, pm))) return rc;
-  for (int t = 0; t < 6; ++t)
-    if ((rc = pass_inverse(c, out.cov[t], CRAVA_GRID_COVARIANCE))) return rc;
+  if ((rc = unit_inverse(c, &out, 3 + c->p.ntheta, 6))) return rc;
   if ((rc = stage_event(c, 3))) return rc;
   c->timed = !c->capture;
   return CRAVA_GPU_OK;
@@ -288,6 +273,8 @@ int crava_gpu_autotune(crava_gpu_ctx *c, const crava_gpu_grids *in, const crava_
   if (tma) cz.insert(cz.begin(), 2);
   const bool xy = plane_xy_supported(c->g);
   for (int lanes = 1; lanes <= 3; ++lanes) {
+    // the built-in passes
+    cand.push_back({-1, -1, 0, 0.0f, lanes, -1, c->consts.kappa_refine, -1, c->consts.solve_shape});
     for (int a : cy)
       for (int z : cz) cand.push_back({a, z, 0, 0.0f, lanes, -1, c->consts.kappa_refine, 0, c->consts.solve_shape});
     // the fused x + y pass replaces the y pass: only the z choices matter

@@ -154,17 +154,80 @@ void prof_collect(crava_gpu_ctx *c) {
   c->recs.clear();
 }
 
-int pass_forward(crava_gpu_ctx *c, const float *src, float *dst, int type, const ZPrior *zp) {
-  int rc;
-  if (use_plane_xy(c->plans)) {
-    { Scope sc(c, K_XY_FWD); if ((rc = plane_xy(c->plans, src, dst, -1, forward_scale(c->g, type), nullptr, c->stream))) return rc; }
-    { Scope sc(c, K_COLS_Z_FWD); if ((rc = fft_cols_z(c->plans, reinterpret_cast<float2 *>(dst), -1, c->stream, zp))) return rc; }
-    return CRAVA_GPU_OK;
+// How n transforms of the built-in passes are spread: grids per launch, and
+// transform lanes (of the context's) they run on.
+//  * A pass over small grids is shorter than a launch, so they share one: all
+//    of them up to 48 MB together, else 24 MB at a time (13 grids of 64x64x128:
+//    92 us per unit in one launch, 96 us in 24 MB launches).
+//  * A grid that with those in flight on the other lanes fits the L2 (126 MB)
+//    goes through its passes there: as many lanes as fit 100 MB (96x200x300, 24
+//    MB: 0.88 ms per unit on 3 lanes against 1.02 ms in one launch per pass;
+//    192x160x384, 48 MB: 1.86 ms on 2 lanes, 1.99 on 3, 1.96 in one launch).
+//  * Larger grids stream from HBM whatever the order: one launch per pass for
+//    all of them has no tails between grids (256x256x512: 4.85 ms per unit
+//    against 5.25 ms on 3 lanes).
+constexpr double kOneLaunch = 48e6, kPerLaunch = 24e6, kInL2 = 100e6;
+struct Spread {
+  int per, lanes;
+};
+Spread spread(const crava_gpu_ctx *c, int n) {
+  const FftPlans &p = c->plans;
+  const int lanes = c->lanes;
+  if (!use_z_batch(p) || !(use_plane(p) || (use_rows_batch(p) && use_y_batch(p)))) return {1, lanes};
+  const double g = (double)c->g.csize * 8.0;
+  const int most = n < kGridBatch ? n : kGridBatch;
+  if (g * n <= kOneLaunch || 2 * g > kInL2) return {most, 1};
+  const int per = g >= kPerLaunch ? 1 : (int)(kPerLaunch / g) < most ? (int)(kPerLaunch / g) : most;
+  const int fit = (int)(kInL2 / (per * g));
+  return {per, fit < lanes ? (fit < 1 ? 1 : fit) : lanes};
+}
+
+// The three passes of the grids of b, forward (b.src -> b.dst) or inverse (in
+// place, + b.add); one launch per pass where it is a built-in one.
+int pass_batch(crava_gpu_ctx *c, const GridBatch &b, int dir, const ZPrior *zp) {
+  const FftPlans &p = c->plans;
+  const double bytes = 2.0 * b.n * (double)c->g.csize * 8.0;
+  int rc = CRAVA_GPU_OK;
+  const bool fused = use_plane(p);
+  auto plane = [&] {
+    Scope sc(c, dir < 0 ? K_XY_FWD : K_XY_INV, bytes);
+    return plane_batch(p, b, dir, c->stream);
+  };
+  auto rows = [&] {
+    Scope sc(c, dir < 0 ? K_ROWS_FWD : K_ROWS_INV, bytes);
+    if (use_rows_batch(p)) return rows_batch(p, b, dir, c->stream);
+    for (int i = 0; i < b.n; ++i)
+      if ((rc = fft_rows(p, b.dst[i], dir, b.scale[i], c->stream, b.add[i], b.src[i]))) return rc;
+    return (int)CRAVA_GPU_OK;
+  };
+  auto y = [&] {
+    Scope sc(c, dir < 0 ? K_COLS_Y_FWD : K_COLS_Y_INV, bytes);
+    if (use_y_batch(p)) return y_batch(p, b, dir, c->stream);
+    for (int i = 0; i < b.n; ++i)
+      if ((rc = fft_cols_y(p, reinterpret_cast<float2 *>(b.dst[i]), dir, c->stream))) return rc;
+    return (int)CRAVA_GPU_OK;
+  };
+  auto z = [&] {
+    Scope sc(c, dir < 0 ? K_COLS_Z_FWD : K_COLS_Z_INV, bytes);
+    if (use_z_batch(p)) return z_batch(p, b, dir, zp, c->stream);
+    for (int i = 0; i < b.n; ++i)
+      if ((rc = fft_cols_z(p, reinterpret_cast<float2 *>(b.dst[i]), dir, c->stream, zp ? zp + i : nullptr))) return rc;
+    return (int)CRAVA_GPU_OK;
+  };
+  if (dir < 0) {
+    if (fused ? (rc = plane()) : (rc = rows()) || (rc = y())) return rc;
+    return z();
   }
-  { Scope sc(c, K_ROWS_FWD); if ((rc = fft_rows(c->plans, dst, -1, forward_scale(c->g, type), c->stream, nullptr, src))) return rc; }
-  { Scope sc(c, K_COLS_Y_FWD); if ((rc = fft_cols_y(c->plans, reinterpret_cast<float2 *>(dst), -1, c->stream))) return rc; }
-  { Scope sc(c, K_COLS_Z_FWD); if ((rc = fft_cols_z(c->plans, reinterpret_cast<float2 *>(dst), -1, c->stream, zp))) return rc; }
-  return CRAVA_GPU_OK;
+  if ((rc = z())) return rc;
+  if (fused) return plane();
+  if ((rc = y())) return rc;
+  return rows();
+}
+
+int pass_forward(crava_gpu_ctx *c, const float *src, float *dst, int type, const ZPrior *zp) {
+  GridBatch b;
+  b.push(src, dst, forward_scale(c->g, type));
+  return pass_batch(c, b, -1, zp);
 }
 
 int gated_prior_setup(crava_gpu_ctx *c, int precision, ZPrior zp[6], bool *on) {
@@ -195,15 +258,9 @@ int gated_prior_count(crava_gpu_ctx *c) {
 }
 
 int pass_inverse(crava_gpu_ctx *c, float *grid, int type, const float *addend) {
-  int rc;
-  { Scope sc(c, K_COLS_Z_INV); if ((rc = fft_cols_z(c->plans, reinterpret_cast<float2 *>(grid), 1, c->stream))) return rc; }
-  if (use_plane_xy(c->plans)) {
-    Scope sc(c, K_XY_INV);
-    return plane_xy(c->plans, grid, grid, 1, inverse_scale(c->g, type), addend, c->stream);
-  }
-  { Scope sc(c, K_COLS_Y_INV); if ((rc = fft_cols_y(c->plans, reinterpret_cast<float2 *>(grid), 1, c->stream))) return rc; }
-  { Scope sc(c, K_ROWS_INV); if ((rc = fft_rows(c->plans, grid, 1, inverse_scale(c->g, type), c->stream, addend))) return rc; }
-  return CRAVA_GPU_OK;
+  GridBatch b;
+  b.push(nullptr, grid, inverse_scale(c->g, type), addend);
+  return pass_batch(c, b, 1, nullptr);
 }
 
 int pass_solve(crava_gpu_ctx *c, const crava_gpu_grids *gr, int precision, bool gated_done) {
@@ -249,15 +306,13 @@ int unit_order(const crava_gpu_ctx *c, const crava_gpu_grids *g, float **ptr, in
   return i;
 }
 
-// Runs `n` independent per-grid steps, step i on lane i % lanes: the lane
-// streams are forked from the context's stream and joined back to it, so
+// Runs `n` independent steps, step i on lane i % lanes: the lane streams are forked from the context's stream and joined back to it, so
 // kernels of different grids (e.g. an ALU-bound x pass and a shared-memory
 // bound z pass) share the SMs.
 template <typename F>
-int on_lanes(crava_gpu_ctx *c, int n, F step) {
-  const int L = c->lanes > 1 && c->lane_s[0]
-                    ? (c->lanes > crava_gpu_ctx::kMaxLanes ? crava_gpu_ctx::kMaxLanes : c->lanes)
-                    : 1;
+int on_lanes(crava_gpu_ctx *c, int n, int lanes, F step) {
+  const int want = lanes < n ? lanes : n;
+  const int L = want > 1 && c->lane_s[0] ? (want > crava_gpu_ctx::kMaxLanes ? crava_gpu_ctx::kMaxLanes : want) : 1;
   if (L == 1) {
     for (int i = 0; i < n; ++i) {
       int rc = step(i);
@@ -281,13 +336,44 @@ int on_lanes(crava_gpu_ctx *c, int n, F step) {
   return rc;
 }
 
+int forward_many(crava_gpu_ctx *c, int n, const float *const *src, float *const *dst, const int *type,
+                 const ZPrior *const *zp) {
+  const Spread sp = spread(c, n);
+  const int per = sp.per, launches = (n + per - 1) / per;
+  auto step = [&](int k) {
+    GridBatch b;
+    ZPrior z[kGridBatch];
+    for (int i = k * per; i < n && b.n < per; ++i) {
+      if (zp && zp[i]) z[b.n] = *zp[i];
+      b.push(src[i], dst[i], forward_scale(c->g, type[i]));
+    }
+    return pass_batch(c, b, -1, z);
+  };
+  return on_lanes(c, launches, sp.lanes, step);
+}
+
+int inverse_many(crava_gpu_ctx *c, int n, float *const *grid, const int *type, const float *const *addend) {
+  const Spread sp = spread(c, n);
+  const int per = sp.per, launches = (n + per - 1) / per;
+  auto step = [&](int k) {
+    GridBatch b;
+    for (int i = k * per; i < n && b.n < per; ++i)
+      b.push(nullptr, grid[i], inverse_scale(c->g, type[i]), addend ? addend[i] : nullptr);
+    return pass_batch(c, b, 1, nullptr);
+  };
+  return on_lanes(c, launches, sp.lanes, step);
+}
+
 int stage_event(crava_gpu_ctx *c, int i) {
   if (!c->capture) CRAVA_CUDA_TRY(cudaEventRecord(c->ev[i], c->stream));
   return CRAVA_GPU_OK;
 }
 
 int inverse_realisations(crava_gpu_ctx *c, float *const *grids, int n, const float *const post_mean[3]) {
-  return on_lanes(c, n, [&](int k) { return pass_inverse(c, grids[k], CRAVA_GRID_PARAMETER, post_mean[k % 3]); });
+  std::vector<int> type(n, CRAVA_GRID_PARAMETER);
+  std::vector<const float *> add(n);
+  for (int k = 0; k < n; ++k) add[k] = post_mean[k % 3];
+  return inverse_many(c, n, grids, type.data(), add.data());
 }
 
 int simulate_batches(crava_gpu_ctx *c, const float2 *const cv[6], const float *const post_mean[3],
@@ -307,10 +393,7 @@ int simulate_batches(crava_gpu_ctx *c, const float2 *const cv[6], const float *c
                                    c->counters, c->stream)))
         return rc;
     }
-    if ((rc = on_lanes(c, 3 * nr, [&](int k) {
-           return pass_inverse(c, out[3 * r0 + k], CRAVA_GRID_PARAMETER, post_mean[k % 3]);
-         })))
-      return rc;
+    if ((rc = inverse_realisations(c, out + 3 * r0, 3 * nr, post_mean))) return rc;
   }
   return CRAVA_GPU_OK;
 }
@@ -357,6 +440,30 @@ int run_unit_fused(crava_gpu_ctx *c, const crava_gpu_grids *in, const crava_gpu_
   return CRAVA_GPU_OK;
 }
 
+int unit_forward(crava_gpu_ctx *c, const crava_gpu_grids *in, const crava_gpu_grids *out, int precision, bool *gated) {
+  float *src[kMaxUnitGrids], *dst[kMaxUnitGrids];
+  int type[kMaxUnitGrids], rc;
+  const int G = unit_order(c, in, src, type);
+  unit_order(c, out, dst, type);
+  // the band-gated bins of the six covariance grids: done by their forward
+  // z passes where the plans allow it, and the solve visits the inverted
+  // planes only
+  ZPrior zp[6];
+  if ((rc = gated_prior_setup(c, precision, zp, gated))) return rc;
+  const int c0 = 3 + c->p.ntheta;  // first covariance grid in unit order
+  const ZPrior *z[kMaxUnitGrids] = {};
+  for (int t = 0; *gated && t < 6; ++t) z[c0 + t] = &zp[t];
+  if ((rc = forward_many(c, G, src, dst, type, z))) return rc;
+  return *gated ? gated_prior_count(c) : (int)CRAVA_GPU_OK;
+}
+
+int unit_inverse(crava_gpu_ctx *c, const crava_gpu_grids *out, int first, int n) {
+  float *dst[kMaxUnitGrids];
+  int type[kMaxUnitGrids];
+  unit_order(c, out, dst, type);
+  return inverse_many(c, n, dst + first, type + first, nullptr);
+}
+
 // The posterior unit reading the real inputs from `in` and leaving the
 // outputs in `out` (in == out is the reference's in-place behaviour).
 int run_unit(crava_gpu_ctx *c, const crava_gpu_grids *in, const crava_gpu_grids *out,
@@ -366,28 +473,13 @@ int run_unit(crava_gpu_ctx *c, const crava_gpu_grids *in, const crava_gpu_grids 
   int rc;
   CRAVA_CUDA_TRY(cudaMemsetAsync(c->counters, 0, sizeof(DevCounters), s));
   if ((rc = stage_event(c, 0))) return rc;
-  float *src[kMaxUnitGrids], *dst[kMaxUnitGrids];
-  int type[kMaxUnitGrids];
-  const int G = unit_order(c, in, src, type);
-  unit_order(c, out, dst, type);
-  // the band-gated bins of the six covariance grids: done by their forward
-  // z passes where the plans allow it, and the solve visits the inverted
-  // planes only
-  ZPrior zp[6];
   bool gated = false;
-  if ((rc = gated_prior_setup(c, precision, zp, &gated))) return rc;
-  const int c0 = 3 + c->p.ntheta;  // first covariance grid in unit order
-  if ((rc = on_lanes(c, G, [&](int i) {
-         const ZPrior *z = gated && i >= c0 && i < c0 + 6 ? &zp[i - c0] : nullptr;
-         return pass_forward(c, src[i], dst[i], type[i], z);
-       })))
-    return rc;
-  if (gated && (rc = gated_prior_count(c))) return rc;
+  if ((rc = unit_forward(c, in, out, precision, &gated))) return rc;
   if ((rc = stage_event(c, 1))) return rc;
   if ((rc = pass_solve(c, out, precision, gated))) return rc;
   if ((rc = stage_event(c, 2))) return rc;
   // the noise correlation (last in unit order) is not an output
-  if ((rc = on_lanes(c, G - 1, [&](int i) { return pass_inverse(c, dst[i], type[i]); }))) return rc;
+  if ((rc = unit_inverse(c, out, 0, 9 + c->p.ntheta))) return rc;
   if ((rc = stage_event(c, 3))) return rc;
   c->timed = !c->capture;
   return CRAVA_GPU_OK;
@@ -544,8 +636,11 @@ int crava_gpu_fft_xy(crava_gpu_ctx *c, float *grid, int dir, int type, int nzp_f
   const Geom full = Geom::make(c->g.nxp, c->g.nyp, nzp_full);
   const float scale = dir < 0 ? forward_scale(full, type) : inverse_scale(full, type);
   int rc;
-  // the same x and y kernels as the 3-D transforms of this geometry
-  if (use_plane_xy(c->plans)) return plane_xy(c->plans, grid, grid, dir, scale, nullptr, c->stream);
+  if (use_plane(c->plans)) {
+    GridBatch b;
+    b.push(grid, grid, scale);
+    return plane_batch(c->plans, b, dir, c->stream);
+  }
   if (dir < 0) {
     if ((rc = fft_rows(c->plans, grid, -1, scale, c->stream))) return rc;
     return fft_cols_y(c->plans, reinterpret_cast<float2 *>(grid), -1, c->stream);

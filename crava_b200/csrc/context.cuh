@@ -99,6 +99,12 @@ bool use_fused(const crava_gpu_ctx *c, int precision);
 int pass_forward(crava_gpu_ctx *c, const float *src, float *dst, int type, const ZPrior *zp = nullptr);
 // Inverse transform in place; addend (optional) is added to the real output.
 int pass_inverse(crava_gpu_ctx *c, float *grid, int type, const float *addend = nullptr);
+// n independent transforms, several per launch where the grids are small,
+// the launches spread over the context's transform lanes.  zp / addend: null
+// or one entry per grid, each null or as in pass_forward / pass_inverse.
+int forward_many(crava_gpu_ctx *c, int n, const float *const *src, float *const *dst, const int *type,
+                 const ZPrior *const *zp);
+int inverse_many(crava_gpu_ctx *c, int n, float *const *grid, const int *type, const float *const *addend);
 // gated_done: the forward z passes applied the band-gated rule (the
 // zp of gated_prior_setup) to the six covariance grids.
 int pass_solve(crava_gpu_ctx *c, const crava_gpu_grids *gr, int precision, bool gated_done = false);
@@ -112,6 +118,11 @@ int gated_prior_count(crava_gpu_ctx *c);
 // Transforms, solve and inverse transforms (in == out: in place).
 int run_unit(crava_gpu_ctx *c, const crava_gpu_grids *in, const crava_gpu_grids *out,
              int precision);
+// The unit's forward transforms (the band-gated rule in them where *gated
+// comes back true), and the inverse transforms of n of its outputs from the
+// first-th on (order: means, residuals, covariances).
+int unit_forward(crava_gpu_ctx *c, const crava_gpu_grids *in, const crava_gpu_grids *out, int precision, bool *gated);
+int unit_inverse(crava_gpu_ctx *c, const crava_gpu_grids *out, int first, int n);
 // Records stage event i on the context's stream (skipped during capture).
 int stage_event(crava_gpu_ctx *c, int i);
 // Inverse transforms of n realisation grids (parameter p = k % 3 of grid

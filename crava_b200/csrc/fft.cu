@@ -798,17 +798,22 @@ int fft_plans_create(const Geom &g, FftPlans *p) {
     CRAVA_CUDA_TRY(cudaMalloc(&p->xpost, sizeof(float2) * (h + 1)));
     CRAVA_CUDA_TRY(cudaMemcpy(p->xpost, post.data(), sizeof(float2) * (h + 1), cudaMemcpyHostToDevice));
   }
-  return plane_xy_tables(g, &p->twq, &p->twy);
+  return pass_plan_create(g, &p->pass);
 }
 
 void fft_plans_destroy(FftPlans *p) {
   cudaFree(p->x.tw); cudaFree(p->y.tw); cudaFree(p->z.tw); cudaFree(p->xpost);
-  cudaFree(p->twq); cudaFree(p->twy);
-  p->x.tw = p->y.tw = p->z.tw = p->xpost = p->twq = p->twy = nullptr;
+  pass_plan_destroy(&p->pass);
+  p->x.tw = p->y.tw = p->z.tw = p->xpost = nullptr;
 }
 
 int fft_rows(const FftPlans &p, float *grid, int dir, float scale, cudaStream_t s,
              const float *addend, const float *src) {
+  if (use_rows_batch(p)) {
+    GridBatch b;
+    b.push(src, grid, scale, addend);
+    return rows_batch(p, b, dir, s);
+  }
   RowArgs a;
   a.addend = addend;
   a.src = src ? src : grid;
@@ -993,46 +998,33 @@ static_assert(RrCols<64>::CPT == 2 && RrCols<512>::CPT == 2 && RrCols<128>::CPT 
 
 int fft_cols_y(const FftPlans &p, float2 *grid, int dir, cudaStream_t s) {
   const Geom &g = p.g;
+  if (use_y_batch(p)) {
+    GridBatch b;
+    b.push(nullptr, reinterpret_cast<float *>(grid), 1.0f);
+    return y_batch(p, b, dir, s);
+  }
   return cols(p.y, grid, g.cnxp, g.cnxp, (long long)g.cnxp * g.nyp, g.nzp, dir, 1.0f, p.tile_y == 2 ? -1 : p.tile_y, s);
 }
 
 bool z_prior_supported(const FftPlans &p) {
-  // the register-resident pass (tile -1 / 1) or its TMA-fed form (2); the
-  // TMA pass falls back to the register-resident one where a grid does not
-  // allow it, which applies the rule too
+  // the built-in pass, else the register-resident pass (tile -1 /
+  // 1) or its TMA-fed form (2; it falls back to the register-resident one
+  // where a grid does not allow it, which applies the rule too)
+  if (use_z_batch(p)) return true;
   return rr::supported(p.g.nzp) && (p.tile_z == -1 || p.tile_z == 1 || p.tile_z == 2);
 }
 
 int fft_cols_z(const FftPlans &p, float2 *grid, int dir, cudaStream_t s, const ZPrior *zp) {
   const Geom &g = p.g;
   if (zp && zp->inv && !z_prior_supported(p)) return CRAVA_GPU_ERR_ARG;
-  // the TMA-fed pass (tile choice 2): faster alone; in the unit's lane
-  // overlap it pays beside the fused x + y pass (5.23 against 5.85 ms per
-  // 256x256x512x5 unit) and not beside the separate passes (5.92 against
-  // 5.40 ms), so it is built in where the fused pass is
-  const bool tma = p.tile_z == 2 || (p.tile_z == -1 && use_plane_xy(p));
-  if (tma && cols_z_tma_supported(g, grid)) return cols_z_tma(p, grid, dir, s, zp);
+  if (use_z_batch(p)) {
+    GridBatch b;
+    b.push(nullptr, reinterpret_cast<float *>(grid), 1.0f);
+    return z_batch(p, b, dir, zp, s);
+  }
+  if (p.tile_z == 2 && cols_z_tma_supported(g, grid)) return cols_z_tma(p, grid, dir, s, zp);
   return cols(p.z, grid, g.cnxp, (long long)g.cnxp * g.nyp, g.cnxp, g.nyp, dir, 1.0f, p.tile_z == 2 ? -1 : p.tile_z, s,
               zp);
-}
-
-int fft3d_r2c(const FftPlans &p, float *grid, int type, cudaStream_t s) {
-  int rc;
-  if (use_plane_xy(p)) {
-    if ((rc = plane_xy(p, grid, grid, -1, forward_scale(p.g, type), nullptr, s))) return rc;
-    return fft_cols_z(p, reinterpret_cast<float2 *>(grid), -1, s);
-  }
-  if ((rc = fft_rows(p, grid, -1, forward_scale(p.g, type), s))) return rc;
-  if ((rc = fft_cols_y(p, reinterpret_cast<float2 *>(grid), -1, s))) return rc;
-  return fft_cols_z(p, reinterpret_cast<float2 *>(grid), -1, s);
-}
-
-int fft3d_c2r(const FftPlans &p, float *grid, int type, cudaStream_t s, const float *addend) {
-  int rc;
-  if ((rc = fft_cols_z(p, reinterpret_cast<float2 *>(grid), 1, s))) return rc;
-  if (use_plane_xy(p)) return plane_xy(p, grid, grid, 1, inverse_scale(p.g, type), addend, s);
-  if ((rc = fft_cols_y(p, reinterpret_cast<float2 *>(grid), 1, s))) return rc;
-  return fft_rows(p, grid, 1, inverse_scale(p.g, type), s, addend);
 }
 
 }  // namespace crava

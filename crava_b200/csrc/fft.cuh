@@ -14,6 +14,31 @@ struct LinePlan {
   float2 *tw = nullptr;
 };
 
+struct ZPrior;
+
+// Grids that one launch of the built-in passes transforms.
+constexpr int kGridBatch = 16;
+struct GridBatch {
+  int n = 0;
+  const float *src[kGridBatch] = {};  // forward: real input (null: dst)
+  float *dst[kGridBatch] = {};
+  const float *add[kGridBatch] = {};  // inverse: real grid added to the output, or null
+  float scale[kGridBatch] = {};
+  void push(const float *from, float *to, float s, const float *addend = nullptr) {
+    src[n] = from; dst[n] = to; scale[n] = s; add[n] = addend;
+    ++n;
+  }
+};
+
+// Tables of the built-in passes (fft_pass.cuh) of the lengths that are
+// compiled: the x line forward and inverse, W_nxp, the y and z lines (null:
+// the length is not compiled, the passes of fft.cu serve it).
+struct PassPlan {
+  float2 *xf = nullptr, *xi = nullptr, *wx = nullptr, *y = nullptr, *z = nullptr;
+  // the fused x + y pass (plane.cu): its y line forward and inverse
+  float2 *pyf = nullptr, *pyi = nullptr;
+};
+
 // Plans of one grid geometry.
 struct FftPlans {
   Geom g;
@@ -34,27 +59,32 @@ struct FftPlans {
   // x pass of an even nxp: -1 default (register-resident where the half
   // length is 64..512), 0 the in-place pass, 1 register-resident
   int rows_x = -1;
-  // x and y passes in one cluster kernel (plane.cu) where the geometry has
-  // one: -1 default (on where the geometry has the kernel), 0 off, 1 on;
-  // its twiddle tables (null where the geometry has none)
+  // x and y passes in one kernel where the geometry has one: -1 default, 0
+  // off, 1 on
   int plane_xy = -1;
-  float2 *twq = nullptr, *twy = nullptr;
+  PassPlan pass;
 };
 
-// The fused x + y pass (plane.cu): geometries with a compiled kernel.
 bool plane_xy_supported(const Geom &g);
-int plane_xy_tables(const Geom &g, float2 **twq, float2 **twy);
-// Forward (dir -1: src real -> dst spectrum in x and y, scaled) or inverse
-// (dir +1: dst spectrum -> dst real, scaled, + addend) x and y passes.
-int plane_xy(const FftPlans &p, const float *src, float *dst, int dir, float scale, const float *addend,
-             cudaStream_t s);
-// Whether the transforms of these plans use the fused x + y pass.
-// Built in where the geometry has the kernel: alone it is slower than the
-// separate register-resident x and y passes (129 / 113 us against 59 + 54 /
-// 56 + 52 us per 256x256x512 grid, forward / inverse), but it moves two
-// grids of HBM traffic instead of four, and in the unit, with the TMA-fed
-// z pass and three transform lanes, it gave 5.23 ms against 5.40 ms.
-inline bool use_plane_xy(const FftPlans &p) { return p.plane_xy != 0 && p.twq && p.twy; }
+// The built-in passes (pass.cu), several grids per launch, in place but for
+// the forward rows (b.src -> b.dst).  zp (forward, optional): one ZPrior per
+// grid, inv null: none.
+int pass_plan_create(const Geom &g, PassPlan *p);
+void pass_plan_destroy(PassPlan *p);
+int rows_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);
+int y_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);
+int z_batch(const FftPlans &p, const GridBatch &b, int dir, const ZPrior *zp, cudaStream_t s);
+int plane_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);  // x and y in one
+// Which passes of these plans they do: where the length is compiled and the
+// tuning names no other.
+inline bool use_rows_batch(const FftPlans &p) { return p.rows_x == -1 && p.pass.xf; }
+inline bool use_y_batch(const FftPlans &p) { return p.tile_y == -1 && p.pass.y; }
+inline bool use_z_batch(const FftPlans &p) { return p.tile_z == -1 && p.pass.z; }
+// The fused x + y pass: where the geometry has it, unless the tuning turns it
+// off or names one of the separate x and y passes (xy_fused 1: on all the same).
+inline bool use_plane(const FftPlans &p) {
+  return p.pass.pyf && (p.plane_xy == 1 || (p.plane_xy == -1 && p.tile_y == -1 && p.rows_x == -1));
+}
 
 // Whether length n has compiled column kernels (tile choices 0, 8, 16).
 bool cols_tunable(int n);
@@ -65,12 +95,6 @@ bool cols_rr(int n);
 bool radix_list(int n, RadixList *out);
 int fft_plans_create(const Geom &g, FftPlans *p);
 void fft_plans_destroy(FftPlans *p);
-
-// In-place transforms of one grid with the FFTGrid scaling of `type`.
-int fft3d_r2c(const FftPlans &p, float *grid, int type, cudaStream_t s);
-// addend (optional): real grid added to the output (posterior mean of a realisation).
-int fft3d_c2r(const FftPlans &p, float *grid, int type, cudaStream_t s,
-              const float *addend = nullptr);
 
 // Individual passes (used by the fused paths).
 // src (forward only, optional): read the real input from src, write grid.

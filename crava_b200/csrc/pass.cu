@@ -1,0 +1,165 @@
+// pass.cu -- host side of the built-in passes (fft_pass.cuh): which lengths
+// are compiled, the stage tables, and the launches.
+#include <math.h>
+
+#include <vector>
+
+#include "fft_pass.cuh"
+
+namespace crava {
+
+#define CRAVA_EIGHTHS(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
+#define CRAVA_DECL(K)           \
+  ColLaunch col_launch_##K(int); \
+  RowLaunch row_launch_##K(int);
+CRAVA_EIGHTHS(CRAVA_DECL)
+#undef CRAVA_DECL
+
+ColLaunch col_launch(int n) {
+#define CRAVA_FIND(K) \
+  if (ColLaunch f = col_launch_##K(n)) return f;
+  CRAVA_EIGHTHS(CRAVA_FIND)
+#undef CRAVA_FIND
+  return nullptr;
+}
+
+RowLaunch row_launch(int nx) {
+#define CRAVA_FIND(K) \
+  if (RowLaunch f = row_launch_##K(nx)) return f;
+  CRAVA_EIGHTHS(CRAVA_FIND)
+#undef CRAVA_FIND
+  return nullptr;
+}
+
+namespace {
+
+int upload(const std::vector<float2> &v, float2 **out) {
+  CRAVA_CUDA_TRY(cudaMalloc(out, sizeof(float2) * v.size()));
+  CRAVA_CUDA_TRY(cudaMemcpy(*out, v.data(), sizeof(float2) * v.size(), cudaMemcpyHostToDevice));
+  return CRAVA_GPU_OK;
+}
+
+float2 root(long long k, int n) {  // e^{-2 pi i k / n}
+  const double ang = -2.0 * M_PI * (double)(k % n) / (double)n;
+  return make_float2((float)cos(ang), (float)sin(ang));
+}
+
+// The stage tables of a line: stage s >= 1, entry q NS + b holds
+// W_n^{q b n / (NS R)}.
+int stage_tables(const LineList &l, int n, float2 **out) {
+  std::vector<float2> t;
+  int ns = l.r[0];
+  for (int s = 1; s < l.n; ++s) {
+    for (int q = 0; q < l.r[s]; ++q)
+      for (int b = 0; b < ns; ++b) t.push_back(root((long long)q * b * (n / (ns * l.r[s])), n));
+    ns *= l.r[s];
+  }
+  return upload(t, out);
+}
+
+// The radices of LineOf<n, pad, desc>.
+LineList line_order(int n, bool pad, bool desc) {
+  LineList l = line_list(n);
+  const bool listed = !pad && (n == 64 || n == 128 || n == 256 || n == 512);
+  if (!listed && l.r[0] != l.r[l.n - 1] && (l.r[0] > l.r[l.n - 1]) != desc)
+    for (int i = 0; i < l.n / 2; ++i) {
+      const int t = l.r[i];
+      l.r[i] = l.r[l.n - 1 - i];
+      l.r[l.n - 1 - i] = t;
+    }
+  return l;
+}
+
+}  // namespace
+
+int pass_plan_create(const Geom &g, PassPlan *p) {
+  int rc;
+  if (row_launch(g.nxp)) {
+    const int n = g.nxp % 2 ? g.nxp : g.nxp / 2;
+    if ((rc = stage_tables(line_order(n, true, false), n, &p->xf)) || (rc = stage_tables(line_order(n, true, true), n, &p->xi))) return rc;
+    std::vector<float2> w(g.nxp / 2 + 1);
+    for (int k = 0; k <= g.nxp / 2; ++k) w[k] = root(k, g.nxp);
+    if ((rc = upload(w, &p->wx))) return rc;
+  }
+  // 32-bit line numbers and offsets in the column passes
+  const bool fits = (long long)g.cnxp * g.nyp < (1LL << 31) && (long long)g.cnxp * g.nzp < (1LL << 31) &&
+                    g.csize < (1LL << 32);
+  if (fits && col_launch(g.nyp) && (rc = stage_tables(line_order(g.nyp, false, true), g.nyp, &p->y))) return rc;
+  if (fits && col_launch(g.nzp) && (rc = stage_tables(line_order(g.nzp, false, true), g.nzp, &p->z))) return rc;
+  if (plane_xy_supported(g)) {
+    // its y line: the stage that holds a column pair first (forward) or last
+    LineList f{}, i{};
+    f.n = i.n = 2;
+    f.r[0] = i.r[1] = 8;
+    f.r[1] = i.r[0] = g.nyp / 8;
+    if ((rc = stage_tables(f, g.nyp, &p->pyf)) || (rc = stage_tables(i, g.nyp, &p->pyi))) return rc;
+  }
+  return CRAVA_GPU_OK;
+}
+
+void pass_plan_destroy(PassPlan *p) {
+  for (float2 **t : {&p->xf, &p->xi, &p->wx, &p->y, &p->z, &p->pyf, &p->pyi}) {
+    cudaFree(*t);
+    *t = nullptr;
+  }
+}
+
+int rows_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) {
+  RowPassArgs a;
+  for (int i = 0; i < b.n; ++i) {
+    a.g.src[i] = dir < 0 && b.src[i] ? b.src[i] : b.dst[i];
+    a.g.dst[i] = b.dst[i];
+    a.g.add[i] = b.add[i];
+    a.g.scale[i] = b.scale[i];
+  }
+  a.nrows = (long long)p.g.nyp * p.g.nzp;
+  a.tw = dir < 0 ? p.pass.xf : p.pass.xi;
+  a.post = p.pass.wx;
+  return row_launch(p.g.nxp)(a, b.n, dir, s);
+}
+
+static ColPassArgs col_args(const GridBatch &b, int dir, const ZPrior *zp) {
+  ColPassArgs a;
+  a.inv = nullptr;
+  a.nf_bits = a.nf_any = nullptr;
+  for (int i = 0; i < b.n; ++i) {
+    a.dst[i] = reinterpret_cast<float2 *>(b.dst[i]);
+    a.mode[i] = 0;
+    a.v[i] = 0.0;
+    if (zp && dir < 0 && zp[i].inv) {
+      a.mode[i] = zp[i].mode;
+      a.v[i] = zp[i].v;
+      a.inv = zp[i].inv;
+      a.nf_bits = zp[i].nf_bits;
+      a.nf_any = zp[i].nf_any;
+    }
+  }
+  return a;
+}
+
+int y_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) {
+  const Geom &g = p.g;
+  ColPassArgs a = col_args(b, dir, nullptr);
+  a.nlines = (long long)g.cnxp * g.nzp;
+  a.inner = (uint32_t)g.cnxp;
+  a.finner = make_fastdiv(a.inner);
+  a.outer = (uint32_t)(g.cnxp * g.nyp);
+  a.es = (uint32_t)g.cnxp;
+  a.tw = p.pass.y;
+  return col_launch(g.nyp)(a, b.n, dir, s);
+}
+
+int z_batch(const FftPlans &p, const GridBatch &b, int dir, const ZPrior *zp, cudaStream_t s) {
+  const Geom &g = p.g;
+  ColPassArgs a = col_args(b, dir, zp);
+  const int plane = g.cnxp * g.nyp;
+  a.nlines = plane;
+  a.inner = (uint32_t)plane;
+  a.finner = make_fastdiv(a.inner);
+  a.outer = 0;
+  a.es = (uint32_t)plane;
+  a.tw = p.pass.z;
+  return col_launch(g.nzp)(a, b.n, dir, s);
+}
+
+}  // namespace crava

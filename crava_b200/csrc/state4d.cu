@@ -469,10 +469,13 @@ int crava_gpu_state4d_advance_time(crava_gpu_ctx *c, const crava_gpu_state4d *st
     return rc;
   // merge: the next prior of the current state, back to the time domain
   if ((rc = crava_gpu_state4d_merge(c, state, mu, cov))) return rc;
-  for (int l = 0; l < 3; ++l)
-    if ((rc = pass_inverse(c, mu[l], CRAVA_GRID_PARAMETER))) return rc;
-  for (int r = 0; r < 6; ++r)
-    if ((rc = pass_inverse(c, cov[r], CRAVA_GRID_COVARIANCE))) return rc;
+  float *grid[9];
+  int type[9];
+  for (int i = 0; i < 9; ++i) {
+    grid[i] = i < 3 ? mu[i] : cov[i - 3];
+    type[i] = i < 3 ? CRAVA_GRID_PARAMETER : CRAVA_GRID_COVARIANCE;
+  }
+  if ((rc = inverse_many(c, 9, grid, type, nullptr))) return rc;
   return read_shortcuts(c, shortcut_bins);
 }
 
