@@ -11,6 +11,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -64,16 +65,18 @@ def build(verbose: bool = False, force: bool = False, extra=()) -> str:
     os.makedirs(os.path.dirname(LIB), exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     headers.append(os.path.join(ROOT, "include", "crava_gpu.h"))
-    objs = []
+    objs, cmds = [], []
     for src, flags in SOURCES.items():
         s = os.path.join(CSRC, src)
         o = os.path.join(OBJ, src.replace(".cu", ".o"))
         objs.append(o)
         if force or _newer(o, [s] + headers):
-            cmd = [NVCC, *ARCH, *FLAGS, *flags, *extra, "-c", s, "-o", o]
+            cmds.append([NVCC, *ARCH, *FLAGS, *flags, *extra, "-c", s, "-o", o])
             if verbose:
-                print(" ".join(cmd), flush=True)
-            subprocess.run(cmd, check=True)
+                print(" ".join(cmds[-1]), flush=True)
+    with ThreadPoolExecutor(max(1, min(8, os.cpu_count() or 1))) as pool:
+        for done in [pool.submit(subprocess.run, cmd, check=True) for cmd in cmds]:
+            done.result()
     if force or _newer(LIB, objs):
         cmd = [NVCC, *ARCH, "-shared", "-cudart", "static", "-o", LIB, *objs]
         if verbose:

@@ -164,8 +164,8 @@ void prof_collect(crava_gpu_ctx *c) {
 //    MB: 0.88 ms per unit on 3 lanes against 1.02 ms in one launch per pass;
 //    192x160x384, 48 MB: 1.86 ms on 2 lanes, 1.99 on 3, 1.96 in one launch).
 //  * Larger grids stream from HBM whatever the order: one launch per pass for
-//    all of them has no tails between grids (256x256x512: 4.85 ms per unit
-//    against 5.25 ms on 3 lanes).
+//    all of them has no tails between grids (256x256x512: 4.90 ms per unit
+//    against 5.03 ms on 3 lanes).
 constexpr double kOneLaunch = 48e6, kPerLaunch = 24e6, kInL2 = 100e6;
 struct Spread {
   int per, lanes;
@@ -191,7 +191,14 @@ int pass_batch(crava_gpu_ctx *c, const GridBatch &b, int dir, const ZPrior *zp) 
   const bool fused = use_plane(p);
   auto plane = [&] {
     Scope sc(c, dir < 0 ? K_XY_FWD : K_XY_INV, bytes);
-    return plane_batch(p, b, dir, c->stream);
+    // a split plane's last y step: in the built-in z pass, else here
+    const bool apart = p.pass.parts > 1 && !use_z_batch(p);
+    for (int i = 0; apart && dir > 0 && i < b.n; ++i)
+      if ((rc = part_radix(p, b.dst[i], dir, c->stream))) return rc;
+    if ((rc = plane_batch(p, b, dir, c->stream))) return rc;
+    for (int i = 0; apart && dir < 0 && i < b.n; ++i)
+      if ((rc = part_radix(p, b.dst[i], dir, c->stream))) return rc;
+    return (int)CRAVA_GPU_OK;
   };
   auto rows = [&] {
     Scope sc(c, dir < 0 ? K_ROWS_FWD : K_ROWS_INV, bytes);
@@ -209,7 +216,7 @@ int pass_batch(crava_gpu_ctx *c, const GridBatch &b, int dir, const ZPrior *zp) 
   };
   auto z = [&] {
     Scope sc(c, dir < 0 ? K_COLS_Z_FWD : K_COLS_Z_INV, bytes);
-    if (use_z_batch(p)) return z_batch(p, b, dir, zp, c->stream);
+    if (use_z_batch(p)) return z_batch(p, b, dir, fused && p.pass.parts > 1, zp, c->stream);
     for (int i = 0; i < b.n; ++i)
       if ((rc = fft_cols_z(p, reinterpret_cast<float2 *>(b.dst[i]), dir, c->stream, zp ? zp + i : nullptr))) return rc;
     return (int)CRAVA_GPU_OK;
@@ -306,9 +313,9 @@ int unit_order(const crava_gpu_ctx *c, const crava_gpu_grids *g, float **ptr, in
   return i;
 }
 
-// Runs `n` independent steps, step i on lane i % lanes: the lane streams are forked from the context's stream and joined back to it, so
-// kernels of different grids (e.g. an ALU-bound x pass and a shared-memory
-// bound z pass) share the SMs.
+// Runs `n` independent steps, step i on lane i % lanes: the lane streams are
+// forked from the context's stream and joined back to it, so kernels of
+// different grids share the SMs.
 template <typename F>
 int on_lanes(crava_gpu_ctx *c, int n, int lanes, F step) {
   const int want = lanes < n ? lanes : n;
@@ -639,7 +646,10 @@ int crava_gpu_fft_xy(crava_gpu_ctx *c, float *grid, int dir, int type, int nzp_f
   if (use_plane(c->plans)) {
     GridBatch b;
     b.push(grid, grid, scale);
-    return plane_batch(c->plans, b, dir, c->stream);
+    const bool parts = c->plans.pass.parts > 1;
+    if (dir > 0 && parts && (rc = part_radix(c->plans, grid, dir, c->stream))) return rc;
+    if ((rc = plane_batch(c->plans, b, dir, c->stream))) return rc;
+    return dir < 0 && parts ? part_radix(c->plans, grid, dir, c->stream) : (int)CRAVA_GPU_OK;
   }
   if (dir < 0) {
     if ((rc = fft_rows(c->plans, grid, -1, scale, c->stream))) return rc;

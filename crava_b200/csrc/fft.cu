@@ -1020,7 +1020,7 @@ int fft_cols_z(const FftPlans &p, float2 *grid, int dir, cudaStream_t s, const Z
   if (use_z_batch(p)) {
     GridBatch b;
     b.push(nullptr, reinterpret_cast<float *>(grid), 1.0f);
-    return z_batch(p, b, dir, zp, s);
+    return z_batch(p, b, dir, false, zp, s);
   }
   if (p.tile_z == 2 && cols_z_tma_supported(g, grid)) return cols_z_tma(p, grid, dir, s, zp);
   return cols(p.z, grid, g.cnxp, (long long)g.cnxp * g.nyp, g.cnxp, g.nyp, dir, 1.0f, p.tile_z == 2 ? -1 : p.tile_z, s,

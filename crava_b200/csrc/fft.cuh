@@ -35,8 +35,10 @@ struct GridBatch {
 // the length is not compiled, the passes of fft.cu serve it).
 struct PassPlan {
   float2 *xf = nullptr, *xi = nullptr, *wx = nullptr, *y = nullptr, *z = nullptr;
-  // the fused x + y pass (plane.cu): its y line forward and inverse
-  float2 *pyf = nullptr, *pyi = nullptr;
+  // the fused x + y pass (plane.cu): CTAs per plane (0: none), its y line
+  // forward and inverse, W_nyp
+  int parts = 0;
+  float2 *pyf = nullptr, *pyi = nullptr, *wy = nullptr;
 };
 
 // Plans of one grid geometry.
@@ -73,8 +75,12 @@ int pass_plan_create(const Geom &g, PassPlan *p);
 void pass_plan_destroy(PassPlan *p);
 int rows_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);
 int y_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);
-int z_batch(const FftPlans &p, const GridBatch &b, int dir, const ZPrior *zp, cudaStream_t s);
-int plane_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);  // x and y in one
+int z_batch(const FftPlans &p, const GridBatch &b, int dir, bool parts, const ZPrior *zp, cudaStream_t s);
+// The fused x + y pass; where it splits a plane (p.pass.parts 2) without the
+// last y step over the parts, which z_batch (parts) or part_radix does.
+int plane_parts(const Geom &g);
+int plane_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);
+int part_radix(const FftPlans &p, float *grid, int dir, cudaStream_t s);
 // Which passes of these plans they do: where the length is compiled and the
 // tuning names no other.
 inline bool use_rows_batch(const FftPlans &p) { return p.rows_x == -1 && p.pass.xf; }
@@ -83,7 +89,7 @@ inline bool use_z_batch(const FftPlans &p) { return p.tile_z == -1 && p.pass.z; 
 // The fused x + y pass: where the geometry has it, unless the tuning turns it
 // off or names one of the separate x and y passes (xy_fused 1: on all the same).
 inline bool use_plane(const FftPlans &p) {
-  return p.pass.pyf && (p.plane_xy == 1 || (p.plane_xy == -1 && p.tile_y == -1 && p.rows_x == -1));
+  return p.pass.parts && (p.plane_xy == 1 || (p.plane_xy == -1 && p.tile_y == -1 && p.rows_x == -1));
 }
 
 // Whether length n has compiled column kernels (tile choices 0, 8, 16).

@@ -13,12 +13,12 @@
 namespace crava {
 
 struct RowBanks {
-  int n, sf, pf, si, pi;  // line length; S and P forward (radices ascending) and inverse (descending)
+  int n, sf, pf, si, pi;  // line length; S and P forward (radices ascending; 32: 8 x 4) and inverse (descending)
 };
 constexpr RowBanks kRowBanks[] = {
     {16, 5, 20, 5, 20}, {18, 7, 21, 5, 35}, {20, 5, 20, 5, 28}, {21, 7, 21, 5, 35},
     {24, 7, 28, 5, 36}, {25, 5, 25, 6, 37}, {27, 11, 33, 3, 35}, {28, 7, 28, 5, 36},
-    {30, 7, 35, 6, 37}, {32, 12, 49, 5, 44}, {35, 11, 55, 6, 53}, {36, 9, 54, 9, 54},
+    {30, 7, 35, 6, 37}, {32, 5, 44, 5, 44}, {35, 11, 55, 6, 53}, {36, 9, 54, 9, 54},
     {40, 9, 45, 6, 53}, {42, 7, 42, 7, 54}, {45, 9, 45, 5, 53}, {48, 9, 54, 6, 54},
     {49, 9, 63, 9, 71}, {50, 13, 65, 5, 53}, {54, 9, 54, 6, 54}, {56, 9, 63, 10, 87},
     {60, 13, 78, 7, 70}, {63, 9, 63, 7, 71}, {64, 9, 72, 9, 72}, {70, 13, 91, 7, 71},

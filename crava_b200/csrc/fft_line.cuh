@@ -96,8 +96,8 @@ struct Dft<9, DIR> {
 template <int DIR> struct Dft<18, DIR> : DftCoprime<2, 9, DIR> {};
 
 // Radices of a length, ascending: as few stages as radices up to 20 allow,
-// the largest radix as small as possible; 64, 128, 256 and 512 take the list
-// of the other passes (CtRadix).  n = 0: none.
+// the largest radix as small as possible; 32, 64, 128, 256 and 512 take the
+// list of the other passes (CtRadix).  n = 0: none.
 struct LineList {
   int n = 0;
   int r[4] = {};
@@ -107,7 +107,7 @@ __host__ __device__ constexpr bool line_radix_ok(int r) {
 }
 __host__ __device__ constexpr LineList line_list(int n) {
   LineList l{};
-  if (n == 64 || n == 128 || n == 256 || n == 512) {
+  if (n == 32 || n == 64 || n == 128 || n == 256 || n == 512) {
     l.n = CtRadix::count(n);
     for (int s = 0; s < l.n; ++s) l.r[s] = CtRadix::at(n, s);
     return l;
@@ -161,14 +161,15 @@ struct CtLine {
   __device__ static __forceinline__ int divM(int x, int s) { return (int)((unsigned)x / (unsigned)M(s)); }
 };
 
-// The line of a length: radices ascending or descending (as listed at 64,
-// 128, 256 and 512 points without padding).
+// The line of a length: radices ascending or descending (as listed at 32, whose
+// x pass so keeps the values of the other x passes, and at 64, 128, 256 and 512
+// points without padding, the y and z passes).
 template <int N, int S0, bool DESC, class I>
 struct LineOfImpl;
 template <int N, int S0, bool DESC, size_t... I>
 struct LineOfImpl<N, S0, DESC, std::index_sequence<I...>> {
   static constexpr LineList kL = line_list(N);
-  static constexpr bool kAsListed = S0 == 0 && (N == 64 || N == 128 || N == 256 || N == 512);
+  static constexpr bool kAsListed = N == 32 || (S0 == 0 && (N == 64 || N == 128 || N == 256 || N == 512));
   static constexpr bool kFlip = !kAsListed && (kL.r[0] > kL.r[kL.n - 1]) != DESC && kL.r[0] != kL.r[kL.n - 1];
   using type = CtLine<S0, kL.r[kFlip ? kL.n - 1 - I : I]...>;
 };

@@ -102,6 +102,27 @@ __device__ __forceinline__ void row_stage(float2 *A, const float2 *tw, int tid) 
   }
 }
 
+// The packed line's values at k and nh - k to the half spectrum's:
+// X_k = E + W^k O, X_{nh-k} = conj(E - W^k O) with E = (z_k + conj z_{nh-k}) / 2,
+// O = -i (z_k - conj z_{nh-k}) / 2; and back (a factor 2 left in):
+// Z_k = e + i o, Z_{nh-k} = conj(e - i o) with e = X_k + conj X_{nh-k},
+// o = conj(W^k) (X_k - conj X_{nh-k}).  Same operations as the other x passes.
+__device__ __forceinline__ void split_pair(float2 zk, float2 zm, float2 w, float2 *xk, float2 *xm) {
+  zm.y = -zm.y;
+  const float2 e = cscale(cadd(zk, zm), 0.5f);
+  const float2 d = csub(zk, zm);
+  const float2 t = cmul(w, make_float2(0.5f * d.y, -0.5f * d.x));
+  *xk = cadd(e, t);
+  *xm = cconj(csub(e, t));
+}
+__device__ __forceinline__ void merge_pair(float2 xk, float2 xm, float2 w, float2 *zk, float2 *zm) {
+  xm.y = -xm.y;
+  const float2 e = cadd(xk, xm);
+  const float2 o = cmul(csub(xk, xm), cconj(w));
+  *zk = make_float2(e.x - o.y, e.y + o.x);
+  *zm = make_float2(e.x + o.y, o.x - e.y);
+}
+
 // Forward rows row0 .. row0 + B of an even nxp: src -> dst (half spectrum).
 template <int NX, int NTH>
 __device__ __forceinline__ void rows_fwd_even(const float *src, float *dst, long long row0, int nrows, float scale,
@@ -136,9 +157,6 @@ __device__ __forceinline__ void rows_fwd_even(const float *src, float *dst, long
     row_stage<L, 2, -1, B, P, NTH>(A, tw, tid);
   }
   __syncthreads();
-  // X_k = (e + T) / 2, X_{nh-k} = conj(e - T) / 2 with e = z_k + conj z_{nh-k},
-  // T = -i W^k (z_k - conj z_{nh-k})
-  const float h = 0.5f * scale;
 #pragma unroll 2
   for (int t = tid; t < B * NP; t += NTH) {
     const int q = t / NP, k = t % NP;
@@ -148,11 +166,10 @@ __device__ __forceinline__ void rows_fwd_even(const float *src, float *dst, long
     const float2 zk = z[line_out(l, k)];
     if (k > 0) {
       const float2 zm = z[line_out(l, NH - k)];
-      const float2 w = __ldg(post + k);
-      const float2 e = make_float2(zk.x + zm.x, zk.y - zm.y);
-      const float2 T = cmul(make_float2(zk.x - zm.x, zk.y + zm.y), make_float2(h * w.y, -(h * w.x)));
-      o[k] = make_float2(h * e.x + T.x, h * e.y + T.y);
-      o[NH - k] = make_float2(h * e.x - T.x, T.y - h * e.y);
+      float2 xk, xm;
+      split_pair(zk, zm, __ldg(post + k), &xk, &xm);
+      o[k] = cscale(xk, scale);
+      o[NH - k] = cscale(xm, scale);
     } else {
       o[0] = make_float2(scale * (zk.x + zk.y), 0.f);
       o[NH] = make_float2(scale * (zk.x - zk.y), 0.f);
@@ -172,9 +189,7 @@ __device__ __forceinline__ void rows_inv_even(const float *src, float *dst, cons
   using L = typename C::I;
   constexpr L l{};
   constexpr int B = C::kB, P = C::PI, NH = C::N, CX = C::CX, NP = C::NP;
-  // Z_k = e + T, Z_{nh-k} = conj(e - T) with e = X_k + conj X_{nh-k},
-  // T = i conj(W^k) (X_k - conj X_{nh-k}); the imaginary parts of the DC and
-  // Nyquist values are ignored
+  // the imaginary parts of the DC and Nyquist values are ignored
   constexpr int G = rounds_group(2, 8, ceil_div(B * NP, NTH));
   float2 xk[G], xm[G], xc[G];
   rounds<B * NP, NTH, G>(
@@ -191,11 +206,7 @@ __device__ __forceinline__ void rows_inv_even(const float *src, float *dst, cons
         const int q = t / NP, k = t % NP;
         float2 *z = A + q * P;
         if (k > 0) {
-          const float2 w = __ldg(post + k);
-          const float2 e = make_float2(xk[u].x + xm[u].x, xk[u].y - xm[u].y);
-          const float2 T = cmul(make_float2(xk[u].x - xm[u].x, xk[u].y + xm[u].y), make_float2(w.y, w.x));
-          z[line_in(l, k)] = cadd(e, T);
-          z[line_in(l, NH - k)] = make_float2(e.x - T.x, T.y - e.y);
+          merge_pair(xk[u], xm[u], __ldg(post + k), z + line_in(l, k), z + line_in(l, NH - k));
         } else {
           z[0] = make_float2(xk[u].x + xm[u].x, xk[u].x - xm[u].x);
           if constexpr (NH % 2 == 0) z[line_in(l, NH / 2)] = make_float2(2.f * xc[u].x, -2.f * xc[u].y);
@@ -532,6 +543,9 @@ int launch_cols(const ColPassArgs &a, int ngrids, cudaStream_t s) {
   CRAVA_LAUNCH_CHECK();
   return CRAVA_GPU_OK;
 }
+
+// The z pass that completes the y transform of planes split in two (plane.cu).
+int z_parts_launch(const ColPassArgs &a, int n, int ngrids, int dir, cudaStream_t s);
 
 // The compiled lengths, each in one of the files fft_len<k>.cu.
 using ColLaunch = int (*)(const ColPassArgs &, int ngrids, int dir, cudaStream_t);

@@ -60,7 +60,7 @@ int stage_tables(const LineList &l, int n, float2 **out) {
 // The radices of LineOf<n, pad, desc>.
 LineList line_order(int n, bool pad, bool desc) {
   LineList l = line_list(n);
-  const bool listed = !pad && (n == 64 || n == 128 || n == 256 || n == 512);
+  const bool listed = n == 32 || (!pad && (n == 64 || n == 128 || n == 256 || n == 512));
   if (!listed && l.r[0] != l.r[l.n - 1] && (l.r[0] > l.r[l.n - 1]) != desc)
     for (int i = 0; i < l.n / 2; ++i) {
       const int t = l.r[i];
@@ -86,19 +86,25 @@ int pass_plan_create(const Geom &g, PassPlan *p) {
                     g.csize < (1LL << 32);
   if (fits && col_launch(g.nyp) && (rc = stage_tables(line_order(g.nyp, false, true), g.nyp, &p->y))) return rc;
   if (fits && col_launch(g.nzp) && (rc = stage_tables(line_order(g.nzp, false, true), g.nzp, &p->z))) return rc;
-  if (plane_xy_supported(g)) {
-    // its y line: the stage that holds a column pair first (forward) or last
+  p->parts = plane_parts(g);
+  if (p->parts) {
+    // the y line of a part: the stage that holds a column pair (radix 8) first
+    // (forward) or last
+    const int nq = g.nyp / p->parts;
     LineList f{}, i{};
     f.n = i.n = 2;
     f.r[0] = i.r[1] = 8;
-    f.r[1] = i.r[0] = g.nyp / 8;
-    if ((rc = stage_tables(f, g.nyp, &p->pyf)) || (rc = stage_tables(i, g.nyp, &p->pyi))) return rc;
+    f.r[1] = i.r[0] = nq / 8;
+    if ((rc = stage_tables(f, nq, &p->pyf)) || (rc = stage_tables(i, nq, &p->pyi))) return rc;
+    std::vector<float2> w(g.nyp);
+    for (int k = 0; k < g.nyp; ++k) w[k] = root(k, g.nyp);
+    if ((rc = upload(w, &p->wy))) return rc;
   }
   return CRAVA_GPU_OK;
 }
 
 void pass_plan_destroy(PassPlan *p) {
-  for (float2 **t : {&p->xf, &p->xi, &p->wx, &p->y, &p->z, &p->pyf, &p->pyi}) {
+  for (float2 **t : {&p->xf, &p->xi, &p->wx, &p->y, &p->z, &p->pyf, &p->pyi, &p->wy}) {
     cudaFree(*t);
     *t = nullptr;
   }
@@ -149,17 +155,17 @@ int y_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) {
   return col_launch(g.nyp)(a, b.n, dir, s);
 }
 
-int z_batch(const FftPlans &p, const GridBatch &b, int dir, const ZPrior *zp, cudaStream_t s) {
+int z_batch(const FftPlans &p, const GridBatch &b, int dir, bool parts, const ZPrior *zp, cudaStream_t s) {
   const Geom &g = p.g;
   ColPassArgs a = col_args(b, dir, zp);
   const int plane = g.cnxp * g.nyp;
-  a.nlines = plane;
+  a.nlines = parts ? plane / p.pass.parts : plane;
   a.inner = (uint32_t)plane;
   a.finner = make_fastdiv(a.inner);
   a.outer = 0;
   a.es = (uint32_t)plane;
   a.tw = p.pass.z;
-  return col_launch(g.nzp)(a, b.n, dir, s);
+  return parts ? z_parts_launch(a, g.nzp, b.n, dir, s) : col_launch(g.nzp)(a, b.n, dir, s);
 }
 
 }  // namespace crava

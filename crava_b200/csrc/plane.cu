@@ -5,27 +5,69 @@ namespace crava {
 
 namespace {
 
-template <int NX, int NY>
+template <int NX, int NY, int CS>
 int launch_plane(const PlaneArgs &a, int dir, int nplanes, int ngrids, cudaStream_t s) {
-  using C = PlaneCfg<NX, NY>;
-  const void *fn = dir < 0 ? (const void *)k_plane_fwd<NX, NY> : (const void *)k_plane_inv<NX, NY>;
+  using C = PlaneCfg<NX, NY, CS>;
+  const void *fn = dir < 0 ? (const void *)k_plane_fwd<NX, NY, CS> : (const void *)k_plane_inv<NX, NY, CS>;
   const size_t smem = C::smem(dir);
   int rc = func_smem(fn, smem);
   if (rc) return rc;
-  const dim3 grd((unsigned)nplanes, (unsigned)ngrids);
-  if (dir < 0) k_plane_fwd<NX, NY><<<grd, C::NTH, smem, s>>>(a);
-  else k_plane_inv<NX, NY><<<grd, C::NTH, smem, s>>>(a);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(nplanes * CS), (unsigned)ngrids);
+  cfg.blockDim = dim3(C::NTH);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = CS;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CS > 1 ? 1 : 0;
+  if (dir < 0) CRAVA_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_plane_fwd<NX, NY, CS>, a));
+  else CRAVA_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_plane_inv<NX, NY, CS>, a));
+  note_launch();
+  return CRAVA_GPU_OK;
+}
+
+template <int N, int CS>
+int launch_parts(const ColPassArgs &a, int ngrids, int dir, cudaStream_t s) {
+  const size_t smem = sizeof(float2) * (size_t)N * kColLines;
+  const void *fn = dir < 0 ? (const void *)k_col_parts<N, -1, CS> : (const void *)k_col_parts<N, 1, CS>;
+  int rc = func_smem(fn, smem);
+  if (rc) return rc;
+  constexpr int TXC = kColLines / CS;
+  const dim3 grd((unsigned)((a.nlines + TXC - 1) / TXC), (unsigned)ngrids);
+  if (dir < 0) k_col_parts<N, -1, CS><<<grd, 256, smem, s>>>(a);
+  else k_col_parts<N, 1, CS><<<grd, 256, smem, s>>>(a);
   CRAVA_LAUNCH_CHECK();
   return CRAVA_GPU_OK;
 }
 
+// The radix-2 step over the parts as a pass of its own (fft_xy).
+template <int DIR>
+__global__ void __launch_bounds__(256) k_part_radix2(float2 *grid, long long part, long long plane) {
+  float2 *g = grid + (long long)blockIdx.y * plane;
+  for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < part; f += (long long)gridDim.x * blockDim.x) {
+    float2 v[2] = {g[f], g[f + part]};
+    Dft<2, DIR>::run(v);
+    g[f] = v[0];
+    g[f + part] = v[1];
+  }
+}
+
 }  // namespace
 
-bool plane_xy_supported(const Geom &g) {
-  // three CTAs per SM: the rows of a plane in 75 KB
+// CTAs per plane; 0: the geometry takes the separate passes.  One where a plane
+// fits 75 KB; two at 256x256 where the z line has the pass that completes y.
+int plane_parts(const Geom &g) {
   const bool px = g.nxp == 64 || g.nxp == 128, py = g.nyp == 64 || g.nyp == 128;
-  return (px && py) || (g.nxp == 256 && g.nyp == 64);
+  if ((px && py) || (g.nxp == 256 && g.nyp == 64)) return 1;
+  const bool z = g.nzp == 64 || g.nzp == 128 || g.nzp == 256 || g.nzp == 512;
+  return g.nxp == 256 && g.nyp == 256 && z ? 2 : 0;
 }
+
+bool plane_xy_supported(const Geom &g) { return plane_parts(g) > 0; }
 
 int plane_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) {
   const Geom &g = p.g;
@@ -39,11 +81,35 @@ int plane_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) 
   a.twx = dir < 0 ? p.pass.xf : p.pass.xi;
   a.twy = dir < 0 ? p.pass.pyf : p.pass.pyi;
   a.wx = p.pass.wx;
-#define CRAVA_PLANE(NX, NY) \
-  if (g.nxp == NX && g.nyp == NY) return launch_plane<NX, NY>(a, dir, g.nzp, b.n, s);
-  CRAVA_PLANE(64, 64) CRAVA_PLANE(64, 128) CRAVA_PLANE(128, 64) CRAVA_PLANE(128, 128) CRAVA_PLANE(256, 64)
+  a.wy = p.pass.wy;
+#define CRAVA_PLANE(NX, NY, CS) \
+  if (g.nxp == NX && g.nyp == NY) return launch_plane<NX, NY, CS>(a, dir, g.nzp, b.n, s);
+  CRAVA_PLANE(64, 64, 1) CRAVA_PLANE(64, 128, 1) CRAVA_PLANE(64, 256, 2)
+  CRAVA_PLANE(128, 64, 1) CRAVA_PLANE(128, 128, 1) CRAVA_PLANE(128, 256, 2)
+  CRAVA_PLANE(256, 64, 1) CRAVA_PLANE(256, 128, 1) CRAVA_PLANE(256, 256, 2)
 #undef CRAVA_PLANE
   return CRAVA_GPU_ERR_ARG;
+}
+
+int z_parts_launch(const ColPassArgs &a, int n, int ngrids, int dir, cudaStream_t s) {
+  switch (n) {
+    case 64: return launch_parts<64, 2>(a, ngrids, dir, s);
+    case 128: return launch_parts<128, 2>(a, ngrids, dir, s);
+    case 256: return launch_parts<256, 2>(a, ngrids, dir, s);
+    case 512: return launch_parts<512, 2>(a, ngrids, dir, s);
+    default: return CRAVA_GPU_ERR_ARG;
+  }
+}
+
+int part_radix(const FftPlans &p, float *real, int dir, cudaStream_t s) {
+  const Geom &g = p.g;
+  float2 *grid = reinterpret_cast<float2 *>(real);
+  const long long plane = (long long)g.cnxp * g.nyp;
+  const dim3 grd(64, (unsigned)g.nzp);
+  if (dir < 0) k_part_radix2<-1><<<grd, 256, 0, s>>>(grid, plane / 2, plane);
+  else k_part_radix2<1><<<grd, 256, 0, s>>>(grid, plane / 2, plane);
+  CRAVA_LAUNCH_CHECK();
+  return CRAVA_GPU_OK;
 }
 
 }  // namespace crava

@@ -1,65 +1,95 @@
-// plane.cuh -- the x and y passes of a 3-D transform in one kernel, for small
-// planes with power-of-two sides: a z-plane lives in a CTA's shared memory
-// between the two passes, three CTAs per SM.
+// plane.cuh -- the x and y passes of a 3-D transform in one kernel, for planes
+// with power-of-two sides: a z-plane, or half of its rows, lives in a CTA's
+// shared memory between the two passes, so a transform moves 4 grids of HBM
+// traffic (this pass and the z pass) where separate x, y and z passes move 6.
+//
+// Planes up to 128x128 are one CTA's (CS = 1; 75 KB, three CTAs per SM).  Of a
+// 256x256 plane CTA r of CS = 2 holds the rows y = CS q + r, q < NQ = nyp / CS
+// (149 KB, 1024 threads).  With ky = k1 + NQ k2,
+//   Y[k1 + NQ k2] = sum_r W_CS^{r k2} [ W_nyp^{r k1} sum_q x[CS q + r] W_NQ^{q k1} ]:
+// the kernel does the brackets, leaves bracket (k1, r) in row k1 + NQ r, and the
+// radix-CS step over r, which needs rows from both CTAs, is the z pass's first
+// butterfly (k_col_parts, 8 adjacent columns of both parts): the rows meet in its
+// registers and cost no extra traffic and no exchange between CTAs.  The inverse
+// runs the same steps backwards.  In place a CTA's output rows are the other
+// CTA's input rows: the two form a cluster, each arrives at its barrier when its
+// loads are done and waits there before its first store.
 //
 // The split of the packed x line into the half spectrum pairs column k with
 // nh - k; the first y stage (forward) or the last one (inverse) takes the two
-// columns of a pair together and does it in registers, so the plane makes three
-// trips through shared memory where the separate passes make three and a trip
-// through L2.  128x128x256, a grid at a time: 12.8 / 12.4 us forward / inverse
-// against 16.8 / 16.7 us for the separate row and column passes.
+// columns of a pair together and does it in registers.
 //
-// Larger planes were tried and are not built: 256x256 split over two CTAs of 150
-// KB (the last radix-2 step of y in the z pass) took 92 + 71 us per transform,
-// over four CTAs of 74 KB 75 + 83 us, and both passes in one cluster kernel with
-// the exchange through L2 104 + 53 us, against 43 + 44 + 52 us for the three
-// separate passes over a batch of grids: those run at the HBM rate, and a CTA
-// that fills the SM has nothing to run while its loads are on the way.
+// Measured, 128x128x256 one grid at a time: 12.8 / 12.4 us forward / inverse
+// (separate row and column passes 16.8 / 16.7 us; the earlier two-CTA cluster
+// kernel 19.0 / 16.7 us).  256x256x512 in a unit of 15 grids, one launch: 83 / 92
+// us and the z pass with the radix-2 step 65 / 60 us, latency-bound (one CTA per
+// SM runs its loads, barriers and stores one after the other).  Against it, per
+// grid: an earlier form over a cluster of four CTAs with the last step through
+// distributed shared memory 108 / 100 us (z 54 / 50); four parts of 74 KB 75 / 74
+// us, but 86 / 80 us in the z pass, whose runs shrink to 32 bytes; both passes
+// in one cluster kernel with the exchange through L2 105 / 103 us; separate row
+// and column passes 43 + 44 / 46 + 51 us at the start of a series, but they draw
+// enough power through the HBM that the clock falls and a unit takes 5.08 ms
+// instead of 4.90.
 #pragma once
 
 #include "fft_pass.cuh"
 
 namespace crava {
 
-template <int NX, int NY>
+template <int NX, int NY, int CS>
 struct PlaneCfg {
-  static constexpr int NH = NX / 2, CX = NH + 1, NP = NH / 2;
+  using R = RowCfg<NX>;
+  static constexpr int NH = NX / 2, CX = NH + 1, NQ = NY / CS, NP = NH / 2;
   static constexpr RowBanks kBanks = row_banks(NH);
   using XF = LineOf<NH, kBanks.sf, false>;
   using XI = LineOf<NH, kBanks.si, true>;
-  // the y line: the stage that holds a column pair has radix 8
-  using YF = CtLine<0, 8, NY / 8>;
-  using YI = CtLine<0, NY / 8, 8>;
+  // the y line: the stage that holds a column pair has the smaller radix
+  using YF = CtLine<0, NQ == 64 ? 8 : NQ == 128 ? 8 : 16, NQ == 64 ? 8 : 16>;
+  using YI = CtLine<0, NQ == 64 ? 8 : 16, NQ == 64 ? 8 : NQ == 128 ? 8 : 16>;
   // a row holds its padded line and a spare slot (the Nyquist column); the
   // pitch keeps the residue that its bank layout wants
   static constexpr int pitch(int line, int want) { return want > line ? want : line + 1 + (want - line - 1 + 1600) % 16; }
   static constexpr int PF = pitch(XF::R(0) * XF::S(0), kBanks.pf), PI = pitch(XI::R(0) * XI::S(0), kBanks.pi);
-  static constexpr size_t smem(int dir) { return sizeof(float2) * (size_t)NY * (dir < 0 ? PF : PI); }
-  static constexpr int NTH = 256;
+  static constexpr size_t smem(int dir) {
+    return sizeof(float2) * ((size_t)NQ * (dir < 0 ? PF : PI) + (CS > 1 ? NQ : 0));
+  }
+  static constexpr int kCtas = 224 * 1024 / (int)(smem(PF > PI ? -1 : 1) + 1024) >= 3 ? 3
+                               : 224 * 1024 / (int)(smem(PF > PI ? -1 : 1) + 1024) >= 2 ? 2 : 1;
+  static constexpr int NTH = kCtas == 3 ? 256 : kCtas == 2 ? 512 : 1024;
+  static constexpr int kMinB = NTH == 256 ? 4 : NTH == 512 ? 2 : 1;
 };
+
+// a s, kept out of the butterflies that follow: contracted into their sums, the
+// product would be rounded in one operand only, and equal rows (the transform
+// of a constant mean) would no longer cancel exactly.
+__device__ __forceinline__ float2 scaled(float2 a, float s) { return make_float2(__fmul_rn(a.x, s), __fmul_rn(a.y, s)); }
 
 struct PlaneArgs {
   PassGrids g;
-  const float2 *twx, *twy, *wx;  // stage tables, W_nxp^k
+  const float2 *twx, *twy, *wx, *wy;  // stage tables, W_nxp^k, W_nyp^k
 };
 
-template <int NX, int NY>
-__global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_fwd(const __grid_constant__ PlaneArgs a) {
-  using C = PlaneCfg<NX, NY>;
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
+
+template <int NX, int NY, int CS>
+__global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS>::kMinB)
+    k_plane_fwd(const __grid_constant__ PlaneArgs a) {
+  using C = PlaneCfg<NX, NY, CS>;
   using LX = typename C::XF;
   using LY = typename C::YF;
   constexpr LX lx{};
   constexpr LY ly{};
-  constexpr int NTH = C::NTH, NQ = NY, NH = C::NH, CX = C::CX, NP = C::NP, P = C::PF, SPARE = LX::R(0) * LX::S(0);
+  constexpr int NTH = C::NTH, NQ = C::NQ, NH = C::NH, CX = C::CX, NP = C::NP, P = C::PF, SPARE = LX::R(0) * LX::S(0);
   static_assert(LX::nst() == 2 && LY::nst() == 2, "two-stage lines");
   extern __shared__ float4 sm4[];
-  float2 *A = reinterpret_cast<float2 *>(sm4);
+  float2 *A = reinterpret_cast<float2 *>(sm4), *twr = A + NQ * P;
   const int tid = threadIdx.x;
-  const int g = blockIdx.y;
-  const long long off = (long long)blockIdx.x * CX * NY;
-  const float2 *src = reinterpret_cast<const float2 *>(a.g.src[g]) + off;
-  float2 *dst = reinterpret_cast<float2 *>(a.g.dst[g]) + off;
-  const float scale = a.g.scale[g], h = 0.5f * scale;
+  const int plane = blockIdx.x / CS, r = blockIdx.x % CS, g = blockIdx.y;
+  const float2 *src = reinterpret_cast<const float2 *>(a.g.src[g]) + (long long)plane * CX * NY + r * CX;
+  float2 *dst = reinterpret_cast<float2 *>(a.g.dst[g]) + (long long)plane * CX * NY + (long long)r * NQ * CX;
+  const float scale = a.g.scale[g];
 
   // 1. x, first stage: HBM -> registers -> shared memory
   {
@@ -68,7 +98,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_fwd(const __
     rounds<NQ * M, NTH, G>(
         tid,
         [&](int u, int t) {
-          const float2 *row = src + (t / M) * CX + t % M;
+          const float2 *row = src + (t / M) * (CS * CX) + t % M;
 #pragma unroll
           for (int i = 0; i < R; ++i) v[u][i] = row[i * M];
         },
@@ -78,6 +108,10 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_fwd(const __
 #pragma unroll
           for (int i = 0; i < R; ++i) o[i * S] = v[u][i];
         });
+  }
+  if constexpr (CS > 1) {
+    for (int k = tid; k < NQ; k += NTH) twr[k] = a.wy[r * k];
+    if (a.g.src[g] == a.g.dst[g]) cluster_arrive();  // this CTA's rows are read
   }
   __syncthreads();
   // 2. x, last stage, in place
@@ -94,24 +128,19 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_fwd(const __
       float2 *om = A + j * P + (k == 0 ? SPARE : line_out(lx, NH - k));
       float2 x[R], y[R];
       if (k > 0) {
-        // e = z_k + conj z_m, T = -i W^k (z_k - conj z_m):
-        // X_k = (e + T) / 2, X_m = conj(e - T) / 2
-        float2 w = __ldg(a.wx + k);
-        w = make_float2(h * w.y, -(h * w.x));
+        const float2 w = __ldg(a.wx + k);
 #pragma unroll
         for (int i = 0; i < R; ++i) {
-          const float2 zk = ok[i * M * P], zm = om[i * M * P];
-          const float2 e = make_float2(zk.x + zm.x, zk.y - zm.y);
-          const float2 T = cmul(make_float2(zk.x - zm.x, zk.y + zm.y), w);
-          x[i] = make_float2(h * e.x + T.x, h * e.y + T.y);
-          y[i] = make_float2(h * e.x - T.x, T.y - h * e.y);
+          split_pair(ok[i * M * P], om[i * M * P], w, &x[i], &y[i]);
+          x[i] = scaled(x[i], scale);
+          y[i] = scaled(y[i], scale);
         }
       } else {
 #pragma unroll
         for (int i = 0; i < R; ++i) {  // DC and Nyquist from z_0
           const float2 z = ok[i * M * P];
-          x[i] = make_float2(scale * (z.x + z.y), 0.f);
-          y[i] = make_float2(scale * (z.x - z.y), 0.f);
+          x[i] = scaled(make_float2(z.x + z.y, 0.f), scale);
+          y[i] = scaled(make_float2(z.x - z.y, 0.f), scale);
         }
       }
       Dft<R, -1>::run(x);
@@ -126,7 +155,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_fwd(const __
 #pragma unroll
         for (int i = 0; i < R; ++i) {
           const float2 z = oc[i * M * P];
-          x[i] = make_float2(scale * z.x, -(scale * z.y));
+          x[i] = scaled(cconj(z), scale);
         }
         Dft<R, -1>::run(x);
 #pragma unroll
@@ -137,6 +166,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_fwd(const __
   __syncthreads();
 
   // 4. y, last stage: shared memory -> registers -> HBM
+  if constexpr (CS > 1) if (a.g.src[g] == a.g.dst[g]) cluster_wait();  // every CTA of the plane has read its rows
   {
     constexpr int R = LY::R(1), M = LY::M(1), S = LY::S(1);
 #pragma unroll 1
@@ -150,28 +180,36 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_fwd(const __
       Dft<R, -1>::run(v);
       float2 *d = dst + j * CX + k;
 #pragma unroll
-      for (int i = 0; i < R; ++i) d[i * M * CX] = v[i];
+      for (int i = 0; i < R; ++i) {
+        if constexpr (CS > 1) d[i * M * CX] = cmul(v[i], twr[j + i * M]);
+        else d[i * M * CX] = v[i];
+      }
     }
   }
 }
 
-template <int NX, int NY>
-__global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_inv(const __grid_constant__ PlaneArgs a) {
-  using C = PlaneCfg<NX, NY>;
+template <int NX, int NY, int CS>
+__global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS>::kMinB)
+    k_plane_inv(const __grid_constant__ PlaneArgs a) {
+  using C = PlaneCfg<NX, NY, CS>;
   using LX = typename C::XI;
   using LY = typename C::YI;
   constexpr LX lx{};
   constexpr LY ly{};
-  constexpr int NTH = C::NTH, NQ = NY, NH = C::NH, CX = C::CX, NP = C::NP, P = C::PI, SPARE = LX::R(0) * LX::S(0);
+  constexpr int NTH = C::NTH, NQ = C::NQ, NH = C::NH, CX = C::CX, NP = C::NP, P = C::PI, SPARE = LX::R(0) * LX::S(0);
   extern __shared__ float4 sm4[];
-  float2 *A = reinterpret_cast<float2 *>(sm4);
+  float2 *A = reinterpret_cast<float2 *>(sm4), *twr = A + NQ * P;
   const int tid = threadIdx.x;
-  const int g = blockIdx.y;
-  const long long off = (long long)blockIdx.x * CX * NY;
-  const float2 *src = reinterpret_cast<const float2 *>(a.g.src[g]) + off;
+  const int plane = blockIdx.x / CS, r = blockIdx.x % CS, g = blockIdx.y;
+  const float2 *src = reinterpret_cast<const float2 *>(a.g.src[g]) + (long long)plane * CX * NY + (long long)r * NQ * CX;
+  const long long off = (long long)plane * CX * NY + r * CX;
   float2 *dst = reinterpret_cast<float2 *>(a.g.dst[g]) + off;
   const float2 *add = a.g.add[g] ? reinterpret_cast<const float2 *>(a.g.add[g]) + off : nullptr;
   const float scale = a.g.scale[g];
+  if constexpr (CS > 1) {
+    for (int k = tid; k < NQ; k += NTH) twr[k] = cconj(a.wy[r * k]);
+    __syncthreads();
+  }
 
   // 1. y, first stage: HBM -> registers -> shared memory
   {
@@ -183,12 +221,17 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_inv(const __
       float2 v[R];
 #pragma unroll
       for (int i = 0; i < R; ++i) v[i] = o[i * M * CX];
+      if constexpr (CS > 1) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) v[i] = cmul(v[i], twr[j + i * M]);
+      }
       Dft<R, 1>::run(v);
       float2 *d = A + j * P + (k == NH ? SPARE : line_in(lx, k));
 #pragma unroll
       for (int i = 0; i < R; ++i) d[i * M * P] = v[i];
     }
   }
+  if constexpr (CS > 1) cluster_arrive();
   __syncthreads();
 
   // 2. y, last stage, and the pre-split of the column pairs, in place
@@ -210,17 +253,9 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_inv(const __
       Dft<R, 1>::run(x);
       Dft<R, 1>::run(y);
       if (k > 0) {
-        // e = X_k + conj X_m, T = i conj(W^k) (X_k - conj X_m):
-        // Z_k = e + T, Z_m = conj(e - T)
-        float2 w = __ldg(a.wx + k);
-        w = make_float2(w.y, w.x);
+        const float2 w = __ldg(a.wx + k);
 #pragma unroll
-        for (int i = 0; i < R; ++i) {
-          const float2 e = make_float2(x[i].x + y[i].x, x[i].y - y[i].y);
-          const float2 T = cmul(make_float2(x[i].x - y[i].x, x[i].y + y[i].y), w);
-          ok[i * S * P] = cadd(e, T);
-          om[i * S * P] = make_float2(e.x - T.x, T.y - e.y);
-        }
+        for (int i = 0; i < R; ++i) merge_pair(x[i], y[i], w, ok + i * S * P, om + i * S * P);
       } else {
         // DC and Nyquist: their imaginary parts are ignored
 #pragma unroll
@@ -241,6 +276,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_inv(const __
   __syncthreads();
 
   // 4. x, last stage: shared memory -> registers -> HBM (scale, addend, zero pad)
+  if constexpr (CS > 1) cluster_wait();
   {
     constexpr int R = LX::R(1), M = LX::M(1), ST = LX::S(1);
 #pragma unroll 1
@@ -249,7 +285,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_inv(const __
       const float2 *o = A + line_out(ly, q) * P + line_slot(lx, 1, j);  // y output q sits in its line's slot
       float2 v[R], w[R];
       if (add) {  // its loads run under the butterfly
-        const float2 *e = add + q * CX + j;
+        const float2 *e = add + q * (CS * CX) + j;
 #pragma unroll
         for (int i = 0; i < R; ++i) w[i] = e[i * M];
       }
@@ -257,7 +293,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_inv(const __
       for (int i = 0; i < R; ++i) v[i] = o[i * ST];
       line_twiddle<R, 1>(lx, 1, j, v, a.twx);
       Dft<R, 1>::run(v);
-      float2 *d = dst + q * CX + j;
+      float2 *d = dst + q * (CS * CX) + j;
       if (add) {
 #pragma unroll
         for (int i = 0; i < R; ++i) d[i * M] = cadd(cscale(v[i], scale), w[i]);
@@ -266,6 +302,142 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY>::NTH, 4) k_plane_inv(const __
         for (int i = 0; i < R; ++i) d[i * M] = cscale(v[i], scale);
       }
       if (j == 0) d[NH] = make_float2(0.f, 0.f);
+    }
+  }
+}
+
+// ------------------------------------------------------------------ z pass of a split plane
+// 16 / CS adjacent columns of all CS parts, rows k1 + NQ r: the radix-CS
+// butterfly over r on registers with the first stage's inputs (forward) or the
+// last stage's outputs (inverse).
+template <int CS>
+__device__ __forceinline__ int swz(int e, int p) { return e * kColLines + ((p + kColLines / CS * e) & (kColLines - 1)); }
+template <int N, int DIR, int CS>
+__global__ void __launch_bounds__(256, 3) k_col_parts(const __grid_constant__ ColPassArgs a) {
+  using L = LineOf<N, 0, true>;
+  constexpr L l{};
+  constexpr int TXC = kColLines / CS, NTH = 256, TPB = NTH / kColLines;
+  extern __shared__ float4 sm4[];
+  float2 *B = reinterpret_cast<float2 *>(sm4);  // [N][kColLines]
+  const int tid = threadIdx.x, g = blockIdx.y;
+  const uint32_t part = (uint32_t)a.nlines, es = a.es;  // lines per part; lines per plane
+  const uint32_t f0 = blockIdx.x * TXC;
+  float2 *data = a.dst[g];
+  const int p = tid % kColLines, t0 = tid / kColLines;
+  const int pc = tid % TXC, tc = tid / TXC;
+  constexpr int TPC = NTH / TXC;
+  const uint32_t line = f0 + p % TXC + (p / TXC) * part;  // of column p of the tile
+  const bool ok = f0 + p % TXC < part, okc = f0 + pc < part;
+  if constexpr (DIR < 0) {
+    constexpr int R = L::R(0), M = L::M(0);
+#pragma unroll 1
+    for (int j = tc; j < M; j += TPC) {
+      if (!okc) break;
+      const uint32_t o = f0 + pc + j * es;
+      float2 v[CS][R];
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int r = 0; r < CS; ++r) v[r][i] = data[o + i * M * es + r * part];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        float2 u[CS];
+#pragma unroll
+        for (int r = 0; r < CS; ++r) u[r] = v[r][i];
+        Dft<CS, -1>::run(u);
+#pragma unroll
+        for (int r = 0; r < CS; ++r) v[r][i] = u[r];
+      }
+#pragma unroll
+      for (int r = 0; r < CS; ++r) {
+        Dft<R, -1>::run(v[r]);
+#pragma unroll
+        for (int i = 0; i < R; ++i) B[swz<CS>(j + i * L::S(0), r * TXC + pc)] = v[r][i];
+      }
+    }
+  } else {
+    constexpr int R = L::R(0), M = L::M(0);
+#pragma unroll 2
+    for (int j = t0; j < M; j += TPB) {
+      if (!ok) break;
+      const uint32_t o = line + j * es;
+      float2 v[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) v[i] = data[o + i * M * es];
+      Dft<R, 1>::run(v);
+#pragma unroll
+      for (int i = 0; i < R; ++i) B[swz<CS>(j + i * L::S(0), p)] = v[i];
+    }
+  }
+  __syncthreads();
+  if constexpr (L::nst() > 2) {
+    constexpr int R = L::R(1), M = L::M(1), ST = L::S(1);
+#pragma unroll 1
+    for (int j = t0; j < M; j += TPB) {
+      const int o = line_slot(l, 1, j);
+      float2 v[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) v[i] = B[swz<CS>(o + i * ST, p)];
+      line_twiddle<R, DIR>(l, 1, j, v, a.tw);
+      Dft<R, DIR>::run(v);
+#pragma unroll
+      for (int i = 0; i < R; ++i) B[swz<CS>(o + i * ST, p)] = v[i];
+    }
+    __syncthreads();
+  }
+  constexpr int S = L::nst() - 1, R = L::R(S), M = L::M(S), ST = L::S(S);
+  if constexpr (DIR < 0) {
+    ZPrior zp;
+    zp.mode = a.mode[g];
+    zp.v = a.v[g];
+    zp.nf_bits = a.nf_bits;
+    zp.nf_any = a.nf_any;
+#pragma unroll 1
+    for (int j = t0; j < M; j += TPB) {
+      if (!ok) break;
+      unsigned gated = 0u;
+      if (zp.mode) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) gated |= __ldg(a.inv + j + i * M) == 0 ? 1u << i : 0u;
+      }
+      const int o = line_slot(l, S, j);
+      float2 v[R];
+#pragma unroll
+      for (int i = 0; i < R; ++i) v[i] = B[swz<CS>(o + i * ST, p)];
+      line_twiddle<R, -1>(l, S, j, v, a.tw);
+      Dft<R, -1>::run(v);
+      if (gated) {
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if ((gated >> i) & 1u) v[i] = zprior_apply(zp, v[i], line + (j + i * M) * es);
+      }
+      const uint32_t d = line + j * es;
+#pragma unroll
+      for (int i = 0; i < R; ++i) data[d + i * M * es] = v[i];
+    }
+  } else {
+#pragma unroll 1
+    for (int j = tc; j < M; j += TPC) {
+      if (!okc) break;
+      const int b = line_slot(l, S, j);
+      float2 v[CS][R];
+#pragma unroll
+      for (int r = 0; r < CS; ++r) {
+#pragma unroll
+        for (int i = 0; i < R; ++i) v[r][i] = B[swz<CS>(b + i * ST, r * TXC + pc)];
+        line_twiddle<R, 1>(l, S, j, v[r], a.tw);
+        Dft<R, 1>::run(v[r]);
+      }
+      const uint32_t d = f0 + pc + j * es;
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        float2 u[CS];
+#pragma unroll
+        for (int r = 0; r < CS; ++r) u[r] = v[r][i];
+        Dft<CS, 1>::run(u);
+#pragma unroll
+        for (int r = 0; r < CS; ++r) data[d + i * M * es + r * part] = u[r];
+      }
     }
   }
 }
