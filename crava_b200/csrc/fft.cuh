@@ -39,6 +39,7 @@ struct PassPlan {
   // forward and inverse, W_nyp
   int parts = 0;
   float2 *pyf = nullptr, *pyi = nullptr, *wy = nullptr;
+  float2 *synt = nullptr;  // the z line of the synthetic seismic (synt_pass.cuh)
 };
 
 // Plans of one grid geometry.

@@ -1,5 +1,5 @@
 // fft_len1.cu -- an eighth of the compiled lengths of the column passes and
-// row sizes of the x pass (fft_pass.cuh): all 2, 3, 5, 7-smooth column lengths
+// of the synthetic seismic, and row sizes of the x pass (fft_pass.cuh): all 2, 3, 5, 7-smooth column lengths
 // 24 .. 512, even rows 32 .. 512 and odd rows 25 .. 255.
 #include "fft_pass.cuh"
 

@@ -20,6 +20,7 @@
 #include "fft.cuh"
 #include "fft_banks.cuh"
 #include "fft_line.cuh"
+#include "synt_pass.cuh"
 
 namespace crava {
 
@@ -562,6 +563,7 @@ int run_rows(const RowPassArgs &a, int ngrids, int dir, cudaStream_t s) {
 }
 #define CRAVA_COL_CASE(N) case N: return run_cols<N>;
 #define CRAVA_ROW_CASE(N) case N: return run_rows<N>;
+#define CRAVA_SYNT_CASE(N) case N: return synt_list(N).n < 2 ? nullptr : run_synt_pass<N>;
 #define CRAVA_LENGTHS(K)                                                    \
   namespace crava {                                                         \
   ColLaunch col_launch_##K(int n) {                                         \
@@ -569,6 +571,9 @@ int run_rows(const RowPassArgs &a, int ngrids, int dir, cudaStream_t s) {
   }                                                                         \
   RowLaunch row_launch_##K(int nx) {                                        \
     switch (nx) { CRAVA_ROWS(CRAVA_ROW_CASE) default: return nullptr; }     \
+  }                                                                         \
+  SyntLaunch synt_launch_##K(int n) {                                       \
+    switch (n) { CRAVA_COLS(CRAVA_SYNT_CASE) default: return nullptr; }     \
   }                                                                         \
   }
 

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "context.cuh"
+#include "synt_pass.cuh"
 
 using namespace crava;
 
@@ -32,164 +33,13 @@ struct SyntArgs {
   const float2 *m[3];     // alpha, beta, rho as float2 pairs
   float2 *out;            // one angle's output grid as float2 pairs
   const float2 *H;        // [nzp] filter of this angle
-  const float2 *tw;       // [nzp] e^{-2 pi i k / nzp}
   float A[3];
   int cnxp, nyp, nzp, nx, ny, nz;
 };
 
-// ((0 + alpha A0) + beta A1) + rho A2 with separate roundings, the
-// reference's float sequence (no fused multiply-add), so the traces the
-// reference leaves unfiltered match it bit for bit.
-__device__ __forceinline__ float imp1(float x, float y, float z, const float *A) {
-  float r = __fadd_rn(0.0f, __fmul_rn(x, A[0]));
-  r = __fadd_rn(r, __fmul_rn(y, A[1]));
-  return __fadd_rn(r, __fmul_rn(z, A[2]));
-}
-
 __device__ __forceinline__ float2 imp_at(const SyntArgs &a, long long idx) {
   const float2 x = a.m[0][idx], y = a.m[1][idx], z = a.m[2][idx];
   return make_float2(imp1(x.x, y.x, z.x, a.A), imp1(x.y, y.y, z.y, a.A));
-}
-
-__device__ __forceinline__ float taper(float v0, float vl, int z, int nz, int nzp) {
-  const float fac = 1.0f / (float)(nzp - nz - 1);
-  return fac * ((float)(z - nz) * v0 + (float)(nzp - z - 1) * vl);
-}
-
-// One CTA: TX complex lines (x pairs x0 .. x0 + TX - 1) at one y, all z.
-template <int N, int TX>
-__global__ void __launch_bounds__(kThreads) k_synt(const __grid_constant__ SyntArgs a) {
-  extern __shared__ float2 sm[];
-  float2 *twl = sm;
-  float2 *buf = twl + N;
-  const int x0 = blockIdx.x * TX, y = blockIdx.y;
-  const int tid = threadIdx.x;
-  const long long plane = (long long)a.cnxp * a.nyp;
-  const long long base = x0 + (long long)a.cnxp * y;
-  for (int i = tid; i < N; i += kThreads) twl[i] = a.tw[i];
-  constexpr int ES = cols_pitch(TX);
-  constexpr int PADR = cols_padr(N, TX);
-  for (int idx = tid; idx < TX * N; idx += kThreads) {
-    const int t = idx % TX, m = idx / TX;
-    buf[pad_row<PADR>(m) * ES + t] = x0 + t < a.cnxp ? imp_at(a, base + m * plane + t) : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  if (y < a.ny && a.nz < N) {
-    for (int idx = tid; idx < TX * (N - a.nz); idx += kThreads) {
-      const int t = idx % TX, m = a.nz + idx / TX;
-      const float2 v0 = buf[t], vl = buf[pad_row<PADR>(a.nz - 1) * ES + t];
-      buf[pad_row<PADR>(m) * ES + t] = make_float2(taper(v0.x, vl.x, m, a.nz, N), taper(v0.y, vl.y, m, a.nz, N));
-    }
-  }
-  __syncthreads();
-  stockham_ip<N, -1, TX, 1, ES, kThreads, PADR>(buf, twl);
-  __syncthreads();
-  for (int idx = tid; idx < TX * N; idx += kThreads) {
-    const int t = idx % TX, m = idx / TX;
-    float2 *b = buf + pad_row<PADR>(m) * ES + t;
-    *b = cmul(*b, __ldg(a.H + m));
-  }
-  __syncthreads();
-  stockham_ip<N, 1, TX, 1, ES, kThreads, PADR>(buf, twl);
-  __syncthreads();
-  for (int idx = tid; idx < TX * N; idx += kThreads) {
-    const int t = idx % TX, m = idx / TX;
-    const int p = x0 + t;
-    if (p >= a.cnxp) continue;
-    const long long g = base + m * plane + t;
-    float2 v = buf[pad_row<PADR>(m) * ES + t];
-    const bool fx = 2 * p < a.nx, fy = 2 * p + 1 < a.nx;
-    if (y >= a.ny || !fx || !fy) {
-      const float2 raw = imp_at(a, g);
-      if (y >= a.ny || !fx) v.x = raw.x;
-      if (y >= a.ny || !fy) v.y = raw.y;
-    }
-    a.out[g] = v;
-  }
-}
-
-// All angles in one pass: a CTA holds its TX lines of the three parameter
-// grids in registers (read from HBM once) and, per angle, forms the
-// impedance in shared memory, tapers, transforms, filters, transforms back
-// and stores: 3 grid reads + nt writes instead of nt (3 reads + 1 write).
-struct SyntAllArgs {
-  const float2 *m[3];
-  float2 *out[CRAVA_GPU_MAX_THETA];
-  const float2 *H;  // [nt][nzp]
-  const float2 *tw;
-  float A[CRAVA_GPU_MAX_THETA][3];
-  int nt, cnxp, nyp, nzp, nx, ny, nz;
-};
-
-template <int N, int TX>
-__global__ void __launch_bounds__(kThreads, N == 256 ? 1 : 2) k_synt_all(const __grid_constant__ SyntAllArgs a) {
-  static_assert((TX * N) % kThreads == 0, "whole elements per thread");
-  constexpr int E = TX * N / kThreads;
-  extern __shared__ float2 sm[];
-  float2 *twl = sm;
-  float2 *buf = twl + N;
-  const int x0 = blockIdx.x * TX, y = blockIdx.y, tid = threadIdx.x;
-  const long long plane = (long long)a.cnxp * a.nyp;
-  const long long base = x0 + (long long)a.cnxp * y;
-  for (int i = tid; i < N; i += kThreads) twl[i] = a.tw[i];
-  float2 pm[3][E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) {
-    const int idx = tid + e * kThreads, t = idx % TX, m = idx / TX;
-    const bool in = x0 + t < a.cnxp;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) pm[q][e] = in ? a.m[q][base + m * plane + t] : make_float2(0.f, 0.f);
-  }
-  for (int l = 0; l < a.nt; ++l) {
-    const float A[3] = {a.A[l][0], a.A[l][1], a.A[l][2]};
-    __syncthreads();  // the previous angle's stores have read buf
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int idx = tid + e * kThreads, t = idx % TX, m = idx / TX;
-      buf[m * TX + t] = make_float2(imp1(pm[0][e].x, pm[1][e].x, pm[2][e].x, A),
-                                    imp1(pm[0][e].y, pm[1][e].y, pm[2][e].y, A));
-    }
-    __syncthreads();
-    if (y < a.ny && a.nz < N) {
-      for (int idx = tid; idx < TX * (N - a.nz); idx += kThreads) {
-        const int t = idx % TX, m = a.nz + idx / TX;
-        const float2 v0 = buf[t], vl = buf[(a.nz - 1) * TX + t];
-        buf[m * TX + t] = make_float2(taper(v0.x, vl.x, m, a.nz, N), taper(v0.y, vl.y, m, a.nz, N));
-      }
-    }
-    __syncthreads();
-    stockham_ip<N, -1, TX, 1, TX, kThreads>(buf, twl);
-    const float2 *H = a.H + (long long)l * N;
-    for (int idx = tid; idx < TX * N; idx += kThreads) {
-      float2 *b = buf + idx;  // (m, t) at m TX + t = idx
-      *b = cmul(*b, __ldg(H + idx / TX));
-    }
-    __syncthreads();
-    stockham_ip<N, 1, TX, 1, TX, kThreads>(buf, twl);
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-      const int idx = tid + e * kThreads, t = idx % TX, m = idx / TX;
-      const int p = x0 + t;
-      if (p >= a.cnxp) continue;
-      float2 v = buf[m * TX + t];
-      const bool fx = 2 * p < a.nx, fy = 2 * p + 1 < a.nx;
-      if (y >= a.ny || !fx) v.x = imp1(pm[0][e].x, pm[1][e].x, pm[2][e].x, A);
-      if (y >= a.ny || !fy) v.y = imp1(pm[0][e].y, pm[1][e].y, pm[2][e].y, A);
-      a.out[l][base + m * plane + t] = v;
-    }
-  }
-}
-
-template <int N>
-int launch_synt_all(const SyntAllArgs &a, cudaStream_t s) {
-  constexpr int TX = 4;
-  const size_t smem = sizeof(float2) * (N + (size_t)TX * N);
-  int rc = func_smem((const void *)k_synt_all<N, TX>, smem);
-  if (rc) return rc;
-  const dim3 grd((unsigned)((a.cnxp + TX - 1) / TX), (unsigned)a.nyp);
-  k_synt_all<N, TX><<<grd, kThreads, smem, s>>>(a);
-  CRAVA_LAUNCH_CHECK();
-  return CRAVA_GPU_OK;
 }
 
 // Generic lengths, step 1: impedance and taper written to the output grid.
@@ -201,11 +51,16 @@ __global__ void __launch_bounds__(kThreads) k_synt_imp(const __grid_constant__ S
   const int m = (int)(idx / plane);
   const long long col = idx - (long long)m * plane;
   const int y = (int)(col / a.cnxp);
-  float2 v = imp_at(a, idx);
-  if (y < a.ny && m >= a.nz) {
-    const float2 v0 = imp_at(a, col), vl = imp_at(a, col + (long long)(a.nz - 1) * plane);
-    v = make_float2(taper(v0.x, vl.x, m, a.nz, a.nzp), taper(v0.y, vl.y, m, a.nz, a.nzp));
-  }
+  // relative to the line's first sample: the filter takes constants to zero,
+  // and what follows then rounds at the size of the line's variation; below
+  // nz the taper fac ((z - nz) imp[0] + (nzp - z - 1) imp[nz - 1])
+  const bool tapered = y < a.ny && m >= a.nz;
+  const long long from = tapered ? col + (long long)(a.nz - 1) * plane : idx;
+  float2 d[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) d[q] = csub(a.m[q][from], a.m[q][col]);
+  float2 v = make_float2(imp1(d[0].x, d[1].x, d[2].x, a.A), imp1(d[0].y, d[1].y, d[2].y, a.A));
+  if (tapered) v = cscale(v, (1.0f / (float)(a.nzp - a.nz - 1)) * (float)(a.nzp - m - 1));
   a.out[idx] = v;
 }
 
@@ -235,18 +90,6 @@ __global__ void __launch_bounds__(kThreads) k_synt_fixup(const __grid_constant__
   a.out[idx] = v;
 }
 
-template <int N>
-int launch_synt(const SyntArgs &a, cudaStream_t s) {
-  constexpr int TX = 8;
-  const size_t smem = sizeof(float2) * (N + (size_t)cols_pitch(TX) * padded_rows(N, cols_padr(N, TX)));
-  int rc = func_smem((const void *)k_synt<N, TX>, smem);
-  if (rc) return rc;
-  const dim3 grd((unsigned)((a.cnxp + TX - 1) / TX), (unsigned)a.nyp);
-  k_synt<N, TX><<<grd, kThreads, smem, s>>>(a);
-  CRAVA_LAUNCH_CHECK();
-  return CRAVA_GPU_OK;
-}
-
 // H_l(kz) = D(kz) conj(W_l(kz)) / nzp in double, stored as float2 [nt][nzp];
 // the upper half is the exact conjugate mirror of the lower, and the kz = 0
 // and Nyquist entries are real (a real-to-complex inverse drops their
@@ -254,15 +97,19 @@ int launch_synt(const SyntArgs &a, cudaStream_t s) {
 std::vector<float2> synt_filters(const crava_gpu_ctx *c) {
   const int nzp = c->p.nzp, nt = c->p.ntheta;
   std::vector<float2> H((size_t)nt * nzp);
+  std::vector<double> cs(nzp), sn(nzp);  // e^{-2 pi i m / nzp}
+  for (int m = 0; m < nzp; ++m) {
+    const double ang = -2.0 * M_PI * (double)m / nzp;
+    cs[m] = cos(ang);
+    sn[m] = sin(ang);
+  }
   for (int l = 0; l < nt; ++l) {
     const float *w = c->wavelet.data() + (size_t)l * nzp;
     for (int k = 0; 2 * k <= nzp; ++k) {
       double wr = 0.0, wi = 0.0;
-      for (int n = 0; n < nzp; ++n) {
-        const long long m = ((long long)k * n) % nzp;
-        const double ang = -2.0 * M_PI * (double)m / nzp;
-        wr += w[n] * cos(ang);
-        wi += w[n] * sin(ang);
+      for (int n = 0, m = 0; n < nzp; ++n, m = m + k < nzp ? m + k : m + k - nzp) {
+        wr += w[n] * cs[m];
+        wi += w[n] * sn[m];
       }
       const double ang = 2.0 * M_PI * (double)k / nzp;
       const double dr = cos(ang) - 1.0, di = sin(ang);
@@ -360,61 +207,46 @@ extern "C" int crava_gpu_synt_seismic(crava_gpu_ctx *c, const float *alpha, cons
     if (cudaMalloc(&c->synt_H, H.size() * sizeof(float2)) != cudaSuccess) { c->synt_H = nullptr; return CRAVA_GPU_ERR_ALLOC; }
     CRAVA_CUDA_TRY(cudaMemcpy(c->synt_H, H.data(), H.size() * sizeof(float2), cudaMemcpyHostToDevice));
   }
+  const cudaStream_t s = c->stream;
+  if (c->plans.pass.synt) {
+    // compiled z lengths: all angles in one pass
+    SyntPassArgs b;
+    b.m[0] = reinterpret_cast<const float2 *>(alpha);
+    b.m[1] = reinterpret_cast<const float2 *>(beta);
+    b.m[2] = reinterpret_cast<const float2 *>(rho);
+    for (int l = 0; l < nt; ++l) {
+      b.out[l] = reinterpret_cast<float2 *>(out[l]);
+      for (int q = 0; q < 3; ++q) b.A[l][q] = c->A[3 * l + q];
+    }
+    b.H = c->synt_H;
+    b.tw = c->plans.pass.synt;
+    b.nt = nt; b.nx = nx; b.ny = ny; b.nz = nz;
+    b.cnxp = (uint32_t)c->g.cnxp;
+    b.plane = (uint32_t)(c->g.cnxp * c->g.nyp);
+    b.fcnxp = make_fastdiv(b.cnxp);
+    return synt_launch(c->g.nzp)(b, s);
+  }
   SyntArgs a{};
   a.m[0] = reinterpret_cast<const float2 *>(alpha);
   a.m[1] = reinterpret_cast<const float2 *>(beta);
   a.m[2] = reinterpret_cast<const float2 *>(rho);
   a.cnxp = c->g.cnxp; a.nyp = c->g.nyp; a.nzp = c->g.nzp;
   a.nx = nx; a.ny = ny; a.nz = nz;
-  a.tw = c->plans.z.tw;
-  const cudaStream_t s = c->stream;
   const long long n = c->g.csize;
   const dim3 eg((unsigned)((n + kThreads - 1) / kThreads));
   int rc;
-  if (c->g.nzp == 128 || c->g.nzp == 256 || c->g.nzp == 512) {
-    SyntAllArgs b{};
-    for (int q = 0; q < 3; ++q) b.m[q] = a.m[q];
-    for (int l = 0; l < nt; ++l) {
-      b.out[l] = reinterpret_cast<float2 *>(out[l]);
-      for (int q = 0; q < 3; ++q) b.A[l][q] = c->A[3 * l + q];
-    }
-    b.H = c->synt_H;
-    b.tw = a.tw;
-    b.nt = nt; b.cnxp = a.cnxp; b.nyp = a.nyp; b.nzp = a.nzp; b.nx = nx; b.ny = ny; b.nz = nz;
-    switch (c->g.nzp) {
-      case 128: return launch_synt_all<128>(b, s);
-      case 256: return launch_synt_all<256>(b, s);
-      default: return launch_synt_all<512>(b, s);
-    }
-  }
   for (int l = 0; l < nt; ++l) {
     a.out = reinterpret_cast<float2 *>(out[l]);
     a.H = c->synt_H + (size_t)l * c->g.nzp;
     for (int q = 0; q < 3; ++q) a.A[q] = c->A[3 * l + q];
-    switch (c->g.nzp) {
-      case 64: rc = launch_synt<64>(a, s); break;
-      case 128: rc = launch_synt<128>(a, s); break;
-      case 256: rc = launch_synt<256>(a, s); break;
-      case 512: rc = launch_synt<512>(a, s); break;
-      case 96: rc = launch_synt<96>(a, s); break;
-      case 160: rc = launch_synt<160>(a, s); break;
-      case 192: rc = launch_synt<192>(a, s); break;
-      case 200: rc = launch_synt<200>(a, s); break;
-      case 300: rc = launch_synt<300>(a, s); break;
-      case 384: rc = launch_synt<384>(a, s); break;
-      default: {
-        k_synt_imp<<<eg, kThreads, 0, s>>>(a);
-        CRAVA_LAUNCH_CHECK();
-        if ((rc = fft_cols_z(c->plans, a.out, -1, s))) return rc;
-        k_synt_filter<<<eg, kThreads, 0, s>>>(a);
-        CRAVA_LAUNCH_CHECK();
-        if ((rc = fft_cols_z(c->plans, a.out, 1, s))) return rc;
-        k_synt_fixup<<<eg, kThreads, 0, s>>>(a);
-        CRAVA_LAUNCH_CHECK();
-        rc = CRAVA_GPU_OK;
-      }
-    }
-    if (rc) return rc;
+    k_synt_imp<<<eg, kThreads, 0, s>>>(a);
+    CRAVA_LAUNCH_CHECK();
+    if ((rc = fft_cols_z(c->plans, a.out, -1, s))) return rc;
+    k_synt_filter<<<eg, kThreads, 0, s>>>(a);
+    CRAVA_LAUNCH_CHECK();
+    if ((rc = fft_cols_z(c->plans, a.out, 1, s))) return rc;
+    k_synt_fixup<<<eg, kThreads, 0, s>>>(a);
+    CRAVA_LAUNCH_CHECK();
   }
   return CRAVA_GPU_OK;
 }

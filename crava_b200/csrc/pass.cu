@@ -11,7 +11,8 @@ namespace crava {
 #define CRAVA_EIGHTHS(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
 #define CRAVA_DECL(K)           \
   ColLaunch col_launch_##K(int); \
-  RowLaunch row_launch_##K(int);
+  RowLaunch row_launch_##K(int); \
+  SyntLaunch synt_launch_##K(int);
 CRAVA_EIGHTHS(CRAVA_DECL)
 #undef CRAVA_DECL
 
@@ -26,6 +27,14 @@ ColLaunch col_launch(int n) {
 RowLaunch row_launch(int nx) {
 #define CRAVA_FIND(K) \
   if (RowLaunch f = row_launch_##K(nx)) return f;
+  CRAVA_EIGHTHS(CRAVA_FIND)
+#undef CRAVA_FIND
+  return nullptr;
+}
+
+SyntLaunch synt_launch(int n) {
+#define CRAVA_FIND(K) \
+  if (SyntLaunch f = synt_launch_##K(n)) return f;
   CRAVA_EIGHTHS(CRAVA_FIND)
 #undef CRAVA_FIND
   return nullptr;
@@ -86,6 +95,7 @@ int pass_plan_create(const Geom &g, PassPlan *p) {
                     g.csize < (1LL << 32);
   if (fits && col_launch(g.nyp) && (rc = stage_tables(line_order(g.nyp, false, true), g.nyp, &p->y))) return rc;
   if (fits && col_launch(g.nzp) && (rc = stage_tables(line_order(g.nzp, false, true), g.nzp, &p->z))) return rc;
+  if (synt_launch(g.nzp) && g.csize < (1LL << 32) && (rc = stage_tables(synt_list(g.nzp), g.nzp, &p->synt))) return rc;
   p->parts = plane_parts(g);
   if (p->parts) {
     // the y line of a part: the stage that holds a column pair (radix 8) first
@@ -104,7 +114,7 @@ int pass_plan_create(const Geom &g, PassPlan *p) {
 }
 
 void pass_plan_destroy(PassPlan *p) {
-  for (float2 **t : {&p->xf, &p->xi, &p->wx, &p->y, &p->z, &p->pyf, &p->pyi, &p->wy}) {
+  for (float2 **t : {&p->xf, &p->xi, &p->wx, &p->y, &p->z, &p->pyf, &p->pyi, &p->wy, &p->synt}) {
     cudaFree(*t);
     *t = nullptr;
   }
