@@ -39,7 +39,9 @@ using namespace crava;
 
 namespace {
 
-constexpr int kThreads = 256;
+// 255 registers: two blocks of 128 threads per SM, so that the planes' shares
+// end within a block's length of each other
+constexpr int kThreads = 128;
 using sb::tri;
 
 __device__ __forceinline__ double2 dconj(double2 a) { return make_double2(a.x, -a.y); }
@@ -58,15 +60,16 @@ struct LLArgs {
   double inv_v[CRAVA_GPU_MAX_THETA];  // 1 / v_l
   int cnxp, nxp;
   long long plane;
-  int bpp;                // blocks per kz plane
-  double *part;           // [nzp][bpp][1 + 4 nt]
+  const int *planes;      // the inverted kz planes (null: every plane, the others skipped)
+  int bpp;                // blocks per visited plane
+  double *part;           // [visited planes][bpp][1 + 4 nt]
   unsigned long long *fail;
 };
 
 template <int NT>
 __global__ void __launch_bounds__(kThreads) k_loglik(const __grid_constant__ LLArgs a) {
   constexpr int NV = 1 + 4 * NT;  // L, g_s[NT], g_v[NT], g_w[NT] (re, im)
-  const int kz = blockIdx.y;
+  const int kz = a.planes ? a.planes[blockIdx.y] : blockIdx.y;
   double acc[NV];
 #pragma unroll
   for (int t = 0; t < NV; ++t) acc[t] = 0.0;
@@ -246,12 +249,25 @@ __global__ void __launch_bounds__(kThreads) k_loglik(const __grid_constant__ LLA
   if (threadIdx.x < NV) {
     double v = 0.0;
     for (int wi = 0; wi < kThreads / 32; ++wi) v += red[wi][threadIdx.x];
-    a.part[((long long)kz * a.bpp + blockIdx.x) * NV + threadIdx.x] = v;
+    a.part[((long long)blockIdx.y * a.bpp + blockIdx.x) * NV + threadIdx.x] = v;
   }
 }
 
-int launch_loglik(const LLArgs &a, int nt, int nzp, cudaStream_t s) {
-  const dim3 grd((unsigned)a.bpp, (unsigned)nzp);
+// The blocks' partial sums of each visited plane in a fixed order: sums[kz][NV]
+// (the other planes' sums were cleared).
+__global__ void __launch_bounds__(64) k_loglik_sum(const double *__restrict__ part, const int *__restrict__ planes, int bpp,
+                                                   int nv, double *__restrict__ sums) {
+  const int v = threadIdx.x;
+  if (v >= nv) return;
+  const int kz = planes ? planes[blockIdx.x] : blockIdx.x;
+  const double *p = part + (long long)blockIdx.x * bpp * nv + v;
+  double s = 0.0;
+  for (int b = 0; b < bpp; ++b) s += p[(long long)b * nv];
+  sums[(long long)kz * nv + v] = s;
+}
+
+int launch_loglik(const LLArgs &a, int nt, int nplanes, cudaStream_t s) {
+  const dim3 grd((unsigned)a.bpp, (unsigned)nplanes);
   switch (nt) {
 #define CRAVA_LL_CASE(N) \
     case N: k_loglik<N><<<grd, kThreads, 0, s>>>(a); break;
@@ -334,21 +350,28 @@ extern "C" int crava_gpu_loglik_grad(crava_gpu_ctx *c, const crava_gpu_grids *gr
   for (int l = 0; l < nt; ++l) { a.inv_s[l] = 1.0 / s[l]; a.inv_v[l] = 1.0 / v[l]; }
   a.cnxp = c->g.cnxp; a.nxp = c->g.nxp;
   a.plane = (long long)c->g.cnxp * c->g.nyp;
+  // Blocks over the inverted planes alone, about four bins per thread where
+  // the grid has enough of them for eight rounds of the device's resident
+  // blocks, else fewer: the last round's idle share stays small
+  // (192x160x384x5: 625 us with two 256-thread blocks for every plane of the
+  // grid, two rounds of which the second was nearly empty).
+  a.planes = c->tables.n_inv > 0 ? c->tables.order_inv : nullptr;
+  const int nplanes = a.planes ? c->tables.n_inv : nzp;
   const long long per_plane_blocks = (a.plane + kThreads - 1) / kThreads;
-  long long bpp = (4LL * 148 + nzp - 1) / nzp;
-  if (bpp > per_plane_blocks) bpp = per_plane_blocks;
-  if (bpp < 1) bpp = 1;
-  a.bpp = (int)bpp;
+  long long bins = per_plane_blocks * nplanes / (8LL * 296);
+  bins = bins < 1 ? 1 : bins > 4 ? 4 : bins;
+  a.bpp = (int)((per_plane_blocks + bins - 1) / bins);
   const int NV = 1 + 4 * nt;
-  const size_t part_n = (size_t)nzp * a.bpp * NV;
-  // the operator table, the partial sums and the failure count live in one
-  // device buffer kept on the context (grown when a call needs more), the
-  // partial sums come back into a pinned host buffer: no allocation, and no
-  // device-wide synchronisation, after the first call
+  const size_t part_n = (size_t)nplanes * a.bpp * NV, sum_n = (size_t)nzp * NV;
+  // the operator table, the partial sums, their per-plane sums and the failure
+  // count live in one device buffer kept on the context (grown when a call
+  // needs more); the per-plane sums and the count come back in one copy into a
+  // pinned host buffer: no allocation after the first call
   const size_t w_bytes = (w.size() * sizeof(double) + 255) / 256 * 256;
   const size_t p_bytes = (part_n * sizeof(double) + 255) / 256 * 256;
-  const size_t need = w_bytes + p_bytes + 256;
-  const size_t host_need = p_bytes + 256;
+  const size_t s_bytes = (sum_n + 1) * sizeof(double);
+  const size_t need = w_bytes + p_bytes + s_bytes;
+  const size_t host_need = s_bytes;
   if (c->ll_bytes < need) {
     cudaFree(c->ll_buf);
     c->ll_buf = nullptr;
@@ -365,39 +388,39 @@ extern "C" int crava_gpu_loglik_grad(crava_gpu_ctx *c, const crava_gpu_grids *gr
   }
   double2 *dw = reinterpret_cast<double2 *>(c->ll_buf);
   double *dpart = reinterpret_cast<double *>(c->ll_buf + w_bytes);
-  unsigned long long *dfail = reinterpret_cast<unsigned long long *>(c->ll_buf + w_bytes + p_bytes);
-  const double *part = reinterpret_cast<const double *>(c->ll_host);
-  const unsigned long long *hfail_p = reinterpret_cast<const unsigned long long *>(c->ll_host + p_bytes);
+  double *dsum = reinterpret_cast<double *>(c->ll_buf + w_bytes + p_bytes);
+  unsigned long long *dfail = reinterpret_cast<unsigned long long *>(dsum + sum_n);
+  const double *sums = reinterpret_cast<const double *>(c->ll_host);
+  const unsigned long long *hfail_p = reinterpret_cast<const unsigned long long *>(sums + sum_n);
   cudaError_t e = cudaMemcpyAsync(dw, w.data(), w.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(dfail, 0, sizeof(unsigned long long), c->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(dsum, 0, s_bytes, c->stream);
   if (e != cudaSuccess) { set_last_error(e, "loglik upload", __FILE__, __LINE__); return CRAVA_GPU_ERR_CUDA; }
   a.w = dw; a.part = dpart; a.fail = dfail;
   // stage events around the kernel: crava_gpu_get_stats then reports its
   // device time as ms_solve and ms_total
   if ((rc = stage_event(c, 0)) || (rc = stage_event(c, 1))) return rc;
-  if ((rc = launch_loglik(a, nt, nzp, c->stream))) return rc;
+  if ((rc = launch_loglik(a, nt, nplanes, c->stream))) return rc;
+  k_loglik_sum<<<nplanes, 64, 0, c->stream>>>(dpart, a.planes, a.bpp, NV, dsum);
+  CRAVA_LAUNCH_CHECK();
   if ((rc = stage_event(c, 2)) || (rc = stage_event(c, 3))) return rc;
   c->timed = true;
-  e = cudaMemcpyAsync(c->ll_host, dpart, part_n * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(c->ll_host + p_bytes, dfail, sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream);
+  e = cudaMemcpyAsync(c->ll_host, dsum, s_bytes, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) { set_last_error(e, "loglik download", __FILE__, __LINE__); return CRAVA_GPU_ERR_CUDA; }
   const unsigned long long hfail = *hfail_p;
   // fixed-order reduction on the host
   double Lsum = 0.0;
   std::vector<double> gs(nt, 0.0), gv(nt, 0.0), gw((size_t)nzp * nt * 2, 0.0);
-  for (int k = 0; k < nzp; ++k)
-    for (int b = 0; b < a.bpp; ++b) {
-      const double *p = &part[((size_t)k * a.bpp + b) * NV];
-      Lsum += p[0];
-      for (int l = 0; l < nt; ++l) {
-        gs[l] += p[1 + l];
-        gv[l] += p[1 + nt + l];
-        gw[((size_t)k * nt + l) * 2] += p[1 + 2 * nt + 2 * l];
-        gw[((size_t)k * nt + l) * 2 + 1] += p[1 + 2 * nt + 2 * l + 1];
-      }
+  for (int k = 0; k < nzp; ++k) {
+    const double *p = sums + (size_t)k * NV;
+    Lsum += p[0];
+    for (int l = 0; l < nt; ++l) {
+      gs[l] += p[1 + l];
+      gv[l] += p[1 + nt + l];
+      gw[((size_t)k * nt + l) * 2] += p[1 + 2 * nt + 2 * l];
+      gw[((size_t)k * nt + l) * 2 + 1] += p[1 + 2 * nt + 2 * l + 1];
     }
+  }
   *loglik = Lsum;
   if (failed_bins) *failed_bins = (long long)hfail;
   if (g_scale) for (int l = 0; l < nt; ++l) g_scale[l] = gs[l];
