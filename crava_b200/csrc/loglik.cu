@@ -75,16 +75,27 @@ __global__ void __launch_bounds__(kThreads) k_loglik(const __grid_constant__ LLA
   for (int t = 0; t < NV; ++t) acc[t] = 0.0;
   unsigned nfail = 0;
   if (a.inv[kz]) {
+    // the plane's constants of M: w_l conj(w_m), theta_lm (e1_l conj(e1_m) +
+    // e2_l conj(e2_m)) and the diagonal wnc theta_ll e3_l^2, formed once per
+    // block (they are a fifth of a bin's arithmetic)
+    __shared__ double2 sW[NT * (NT + 1) / 2], sE[NT * (NT + 1) / 2];
+    __shared__ double sD[NT];
     double2 w[NT];
-    float2 e1[NT], e2[NT];
-    float e3[NT];
 #pragma unroll
-    for (int l = 0; l < NT; ++l) {
-      w[l] = a.w[(long long)kz * NT + l];
-      e1[l] = a.e1[(long long)kz * NT + l];
-      e2[l] = a.e2[(long long)kz * NT + l];
-      e3[l] = a.e3[(long long)kz * NT + l];
+    for (int l = 0; l < NT; ++l) w[l] = a.w[(long long)kz * NT + l];
+    for (int t = threadIdx.x; t < NT * NT; t += kThreads) {
+      const int l = t / NT, m = t % NT;
+      if (m > l) continue;
+      const long long o = (long long)kz * NT;
+      const float2 p1 = a.e1[o + l], q1 = a.e1[o + m], p2 = a.e2[o + l], q2 = a.e2[o + m];
+      const double2 n1 = dmulc(make_double2(p1.x, p1.y), make_double2(q1.x, q1.y));
+      const double2 n2 = dmulc(make_double2(p2.x, p2.y), make_double2(q2.x, q2.y));
+      sW[tri(l, m)] = dmulc(a.w[o + l], a.w[o + m]);
+      sE[tri(l, m)] = make_double2(a.c.theta[l][m] * (n1.x + n2.x), a.c.theta[l][m] * (n1.y + n2.y));
+      const double e3 = a.e3[o + l];
+      if (m == l) sD[l] = (double)a.c.wnc * a.c.theta[l][l] * e3 * e3;
     }
+    __syncthreads();
     const SolveConsts &c = a.c;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < a.plane;
          i += (long long)a.bpp * blockDim.x) {
@@ -132,13 +143,10 @@ __global__ void __launch_bounds__(kThreads) k_loglik(const __grid_constant__ LLA
         for (int m = 0; m <= l; ++m) {
           const double b = as0 * c.A[m][0] + as1 * c.A[m][1] + as2 * c.A[m][2];
           B[tri(l, m)] = b;
-          const double2 ww = dmulc(w[l], w[m]);
-          const double2 n1 = dmulc(make_double2(e1[l].x, e1[l].y), make_double2(e1[m].x, e1[m].y));
-          const double2 n2 = dmulc(make_double2(e2[l].x, e2[l].y), make_double2(e2[m].x, e2[m].y));
-          const double f = cc * c.theta[l][m];
-          double2 v = make_double2(ww.x * b + f * (n1.x + n2.x), ww.y * b + f * (n1.y + n2.y));
+          const double2 ww = sW[tri(l, m)], ee = sE[tri(l, m)];
+          double2 v = make_double2(ww.x * b + cc * ee.x, ww.y * b + cc * ee.y);
           if (l == m) {
-            v.x += (double)c.wnc * c.theta[l][l] * (double)e3[l] * (double)e3[l];
+            v.x += sD[l];
             v.y = 0.0;
           }
           L[tri(l, m)] = v;
@@ -209,19 +217,8 @@ __global__ void __launch_bounds__(kThreads) k_loglik(const __grid_constant__ LLA
           const double2 cw = make_double2(w[m].x * b, -w[m].y * b);  // conj(w_m) B_lm
           u = dadd(u, dmul(Gml, cw));
           // N_lm (row l = j of the noise gradient)
-          double2 n;
-          if (m == l) {
-            n = make_double2(cc * c.theta[l][l] *
-                                 ((double)e1[l].x * e1[l].x + (double)e1[l].y * e1[l].y +
-                                  (double)e2[l].x * e2[l].x + (double)e2[l].y * e2[l].y) +
-                             (double)c.wnc * c.theta[l][l] * (double)e3[l] * (double)e3[l],
-                             0.0);
-          } else {
-            const double2 n1 = dmulc(make_double2(e1[l].x, e1[l].y), make_double2(e1[m].x, e1[m].y));
-            const double2 n2 = dmulc(make_double2(e2[l].x, e2[l].y), make_double2(e2[m].x, e2[m].y));
-            const double f = cc * c.theta[l][m];
-            n = make_double2(f * (n1.x + n2.x), f * (n1.y + n2.y));
-          }
+          const double2 ee = m >= l ? dconj(sE[tri(m, l)]) : sE[tri(l, m)];
+          const double2 n = make_double2(cc * ee.x + (m == l ? sD[l] : 0.0), m == l ? 0.0 : cc * ee.y);
           gv += Gml.x * n.x - Gml.y * n.y;  // Re(G_ml N_lm)
         }
         acc[1 + l] += ck * 2.0 * (w[l].x * u.x - w[l].y * u.y) * a.inv_s[l];
