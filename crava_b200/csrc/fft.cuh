@@ -34,6 +34,7 @@ struct GridBatch {
 // compiled: the x line forward and inverse, W_nxp, the y and z lines (null:
 // the length is not compiled, the passes of fft.cu serve it).
 struct PassPlan {
+  float2 *tables = nullptr;  // one buffer; the pointers below lie in it
   float2 *xf = nullptr, *xi = nullptr, *wx = nullptr, *y = nullptr, *z = nullptr;
   // the fused x + y pass (plane.cu): CTAs per plane (0: none), its y line
   // forward and inverse, W_nyp

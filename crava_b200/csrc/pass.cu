@@ -42,11 +42,16 @@ SyntLaunch synt_launch(int n) {
 
 namespace {
 
-int upload(const std::vector<float2> &v, float2 **out) {
-  CRAVA_CUDA_TRY(cudaMalloc(out, sizeof(float2) * v.size()));
-  CRAVA_CUDA_TRY(cudaMemcpy(*out, v.data(), sizeof(float2) * v.size(), cudaMemcpyHostToDevice));
-  return CRAVA_GPU_OK;
-}
+// Tables of one geometry, gathered on the host and uploaded in one copy: the
+// pointers are set when the device buffer exists.
+struct Tables {
+  std::vector<float2> host;
+  std::vector<std::pair<float2 **, size_t>> at;
+  void add(const std::vector<float2> &v, float2 **out) {
+    at.emplace_back(out, host.size());
+    host.insert(host.end(), v.begin(), v.end());
+  }
+};
 
 float2 root(long long k, int n) {  // e^{-2 pi i k / n}
   const double ang = -2.0 * M_PI * (double)(k % n) / (double)n;
@@ -55,7 +60,7 @@ float2 root(long long k, int n) {  // e^{-2 pi i k / n}
 
 // The stage tables of a line: stage s >= 1, entry q NS + b holds
 // W_n^{q b n / (NS R)}.
-int stage_tables(const LineList &l, int n, float2 **out) {
+void stage_tables(const LineList &l, int n, Tables *to, float2 **out) {
   std::vector<float2> t;
   int ns = l.r[0];
   for (int s = 1; s < l.n; ++s) {
@@ -63,7 +68,7 @@ int stage_tables(const LineList &l, int n, float2 **out) {
       for (int b = 0; b < ns; ++b) t.push_back(root((long long)q * b * (n / (ns * l.r[s])), n));
     ns *= l.r[s];
   }
-  return upload(t, out);
+  to->add(t, out);
 }
 
 // The radices of LineOf<n, pad, desc>.
@@ -82,20 +87,24 @@ LineList line_order(int n, bool pad, bool desc) {
 }  // namespace
 
 int pass_plan_create(const Geom &g, PassPlan *p) {
-  int rc;
+  Tables t;
+  auto roots = [&](int n, int count, float2 **out) {
+    std::vector<float2> w(count);
+    for (int k = 0; k < count; ++k) w[k] = root(k, n);
+    t.add(w, out);
+  };
   if (row_launch(g.nxp)) {
     const int n = g.nxp % 2 ? g.nxp : g.nxp / 2;
-    if ((rc = stage_tables(line_order(n, true, false), n, &p->xf)) || (rc = stage_tables(line_order(n, true, true), n, &p->xi))) return rc;
-    std::vector<float2> w(g.nxp / 2 + 1);
-    for (int k = 0; k <= g.nxp / 2; ++k) w[k] = root(k, g.nxp);
-    if ((rc = upload(w, &p->wx))) return rc;
+    stage_tables(line_order(n, true, false), n, &t, &p->xf);
+    stage_tables(line_order(n, true, true), n, &t, &p->xi);
+    roots(g.nxp, g.nxp / 2 + 1, &p->wx);
   }
   // 32-bit line numbers and offsets in the column passes
   const bool fits = (long long)g.cnxp * g.nyp < (1LL << 31) && (long long)g.cnxp * g.nzp < (1LL << 31) &&
                     g.csize < (1LL << 32);
-  if (fits && col_launch(g.nyp) && (rc = stage_tables(line_order(g.nyp, false, true), g.nyp, &p->y))) return rc;
-  if (fits && col_launch(g.nzp) && (rc = stage_tables(line_order(g.nzp, false, true), g.nzp, &p->z))) return rc;
-  if (synt_launch(g.nzp) && g.csize < (1LL << 32) && (rc = stage_tables(synt_list(g.nzp), g.nzp, &p->synt))) return rc;
+  if (fits && col_launch(g.nyp)) stage_tables(line_order(g.nyp, false, true), g.nyp, &t, &p->y);
+  if (fits && col_launch(g.nzp)) stage_tables(line_order(g.nzp, false, true), g.nzp, &t, &p->z);
+  if (fits && synt_launch(g.nzp)) stage_tables(synt_list(g.nzp), g.nzp, &t, &p->synt);
   p->parts = plane_parts(g);
   if (p->parts) {
     // the y line of a part: the stage that holds a column pair (radix 8) first
@@ -105,19 +114,21 @@ int pass_plan_create(const Geom &g, PassPlan *p) {
     f.n = i.n = 2;
     f.r[0] = i.r[1] = 8;
     f.r[1] = i.r[0] = nq / 8;
-    if ((rc = stage_tables(f, nq, &p->pyf)) || (rc = stage_tables(i, nq, &p->pyi))) return rc;
-    std::vector<float2> w(g.nyp);
-    for (int k = 0; k < g.nyp; ++k) w[k] = root(k, g.nyp);
-    if ((rc = upload(w, &p->wy))) return rc;
+    stage_tables(f, nq, &t, &p->pyf);
+    stage_tables(i, nq, &t, &p->pyi);
+    roots(g.nyp, g.nyp, &p->wy);
   }
+  if (t.host.empty()) return CRAVA_GPU_OK;
+  const size_t bytes = sizeof(float2) * t.host.size();
+  CRAVA_CUDA_TRY(cudaMalloc(&p->tables, bytes));
+  CRAVA_CUDA_TRY(cudaMemcpy(p->tables, t.host.data(), bytes, cudaMemcpyHostToDevice));
+  for (auto &e : t.at) *e.first = p->tables + e.second;
   return CRAVA_GPU_OK;
 }
 
 void pass_plan_destroy(PassPlan *p) {
-  for (float2 **t : {&p->xf, &p->xi, &p->wx, &p->y, &p->z, &p->pyf, &p->pyi, &p->wy, &p->synt}) {
-    cudaFree(*t);
-    *t = nullptr;
-  }
+  cudaFree(p->tables);
+  *p = PassPlan{};
 }
 
 int rows_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) {
