@@ -84,9 +84,9 @@ int plane_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) 
   a.wy = p.pass.wy;
 #define CRAVA_PLANE(NX, NY, CS) \
   if (g.nxp == NX && g.nyp == NY) return launch_plane<NX, NY, CS>(a, dir, g.nzp, b.n, s);
-  CRAVA_PLANE(64, 64, 1) CRAVA_PLANE(64, 128, 1) CRAVA_PLANE(64, 256, 2)
-  CRAVA_PLANE(128, 64, 1) CRAVA_PLANE(128, 128, 1) CRAVA_PLANE(128, 256, 2)
-  CRAVA_PLANE(256, 64, 1) CRAVA_PLANE(256, 128, 1) CRAVA_PLANE(256, 256, 2)
+  CRAVA_PLANE(64, 64, 1) CRAVA_PLANE(64, 128, 1)
+  CRAVA_PLANE(128, 64, 1) CRAVA_PLANE(128, 128, 1)
+  CRAVA_PLANE(256, 64, 1) CRAVA_PLANE(256, 256, 2)
 #undef CRAVA_PLANE
   return CRAVA_GPU_ERR_ARG;
 }
