@@ -388,6 +388,7 @@ struct ColPassArgs {
   int mode[kGridBatch];
   const int *inv;
   unsigned *nf_bits, *nf_any;
+  uint32_t ahead;  // z pass of split planes: tiles ahead whose input is fetched into L2
 };
 
 template <int N>

@@ -5,13 +5,22 @@ namespace crava {
 
 namespace {
 
+int sm_count(int *n) {
+  int dev = 0;
+  CRAVA_CUDA_TRY(cudaGetDevice(&dev));
+  CRAVA_CUDA_TRY(cudaDeviceGetAttribute(n, cudaDevAttrMultiProcessorCount, dev));
+  return CRAVA_GPU_OK;
+}
+
 template <int NX, int NY, int CS>
-int launch_plane(const PlaneArgs &a, int dir, int nplanes, int ngrids, cudaStream_t s) {
+int launch_plane(PlaneArgs a, int dir, int nplanes, int ngrids, cudaStream_t s) {
   using C = PlaneCfg<NX, NY, CS>;
   const void *fn = dir < 0 ? (const void *)k_plane_fwd<NX, NY, CS> : (const void *)k_plane_inv<NX, NY, CS>;
   const size_t smem = C::smem(dir);
   int rc = func_smem(fn, smem);
   if (rc) return rc;
+  a.ahead = 0;
+  if (CS > 1 && (rc = sm_count(&a.ahead))) return rc;  // one CTA per SM
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(nplanes * CS), (unsigned)ngrids);
   cfg.blockDim = dim3(C::NTH);
@@ -31,11 +40,12 @@ int launch_plane(const PlaneArgs &a, int dir, int nplanes, int ngrids, cudaStrea
 }
 
 template <int N, int CS>
-int launch_parts(const ColPassArgs &a, int ngrids, int dir, cudaStream_t s) {
+int launch_parts(ColPassArgs a, int ngrids, int dir, cudaStream_t s) {
   const size_t smem = sizeof(float2) * (size_t)N * kColLines;
   const void *fn = dir < 0 ? (const void *)k_col_parts<N, -1, CS> : (const void *)k_col_parts<N, 1, CS>;
-  int rc = func_smem(fn, smem);
-  if (rc) return rc;
+  int sms = 0, rc = func_smem(fn, smem);
+  if (rc || (rc = sm_count(&sms))) return rc;
+  a.ahead = (uint32_t)(7 * sms / 4);  // of 3 resident per SM; see fetch_l2
   constexpr int TXC = kColLines / CS;
   const dim3 grd((unsigned)((a.nlines + TXC - 1) / TXC), (unsigned)ngrids);
   if (dir < 0) k_col_parts<N, -1, CS><<<grd, 256, smem, s>>>(a);

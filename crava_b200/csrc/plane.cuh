@@ -21,16 +21,17 @@
 //
 // Measured, 128x128x256 one grid at a time: 12.8 / 12.4 us forward / inverse
 // (separate row and column passes 16.8 / 16.7 us; the earlier two-CTA cluster
-// kernel 19.0 / 16.7 us).  256x256x512 in a unit of 15 grids, one launch: 83 / 92
-// us and the z pass with the radix-2 step 65 / 60 us, latency-bound (one CTA per
-// SM runs its loads, barriers and stores one after the other).  Against it, per
-// grid: an earlier form over a cluster of four CTAs with the last step through
-// distributed shared memory 108 / 100 us (z 54 / 50); four parts of 74 KB 75 / 74
-// us, but 86 / 80 us in the z pass, whose runs shrink to 32 bytes; both passes
-// in one cluster kernel with the exchange through L2 105 / 103 us; separate row
-// and column passes 43 + 44 / 46 + 51 us at the start of a series, but they draw
-// enough power through the HBM that the clock falls and a unit takes 5.08 ms
-// instead of 4.90.
+// kernel 19.0 / 16.7 us).  256x256x512 in a unit of 15 grids, one launch: 81 / 85
+// us and the z pass with the radix-2 step 53 / 50 us (41 us at the copy rate);
+// one CTA per SM runs its loads, barriers and stores one after the other, with
+// the next CTA's input on its way into L2 meanwhile (fetch_l2).  Against it, per
+// grid and before that fetch (88 / 93, z 66 / 61): an earlier form over a cluster
+// of four CTAs with the last step through distributed shared memory 108 / 100 us
+// (z 54 / 50); four parts of 74 KB 75 / 74 us, but 86 / 80 us in the z pass, whose
+// runs shrink to 32 bytes; both passes in one cluster kernel with the exchange
+// through L2 105 / 103 us; separate row and column passes 43 + 44 / 46 + 51 us at
+// the start of a series, but they draw enough power through the HBM that the
+// clock falls and a unit takes 5.08 ms instead of 4.90 (4.47 with the fetch).
 #pragma once
 
 #include "fft_pass.cuh"
@@ -68,7 +69,36 @@ __device__ __forceinline__ float2 scaled(float2 a, float s) { return make_float2
 struct PlaneArgs {
   PassGrids g;
   const float2 *twx, *twy, *wx, *wy;  // stage tables, W_nxp^k, W_nyp^k
+  int ahead;                          // CTAs ahead whose input is fetched into L2 (CS > 1)
 };
+
+// With one CTA per SM nothing runs under a CTA's loads, so it asks for the data
+// of the CTA that will take its place, one wave on, as soon as its own loads are
+// done: HBM then works under its butterflies and stores, and the next loads find
+// their lines in L2 (a wave's reads are 20 MB).  256x256x512, a unit of 15 grids
+// in one launch, per grid: 88 / 93 -> 81 / 85 us forward / inverse, and the z
+// pass of the parts (k_col_parts) 66 / 61 -> 53 / 50.  Half the wave ahead or the
+// wave: the same in the plane passes; 1.75 CTAs per SM ahead of 3 resident are
+// best in the z pass (2 and 1.5 per SM 54 / 50 and 54 / 52, 3 per SM 57 / 53, 1
+// per SM 58 / 58, 6 per SM 70 / 68).  In
+// the row and column passes of smaller grids (several CTAs per SM, inputs mostly
+// in L2) nothing is gained: within 1 % at 1 to 4 per SM.
+__device__ __forceinline__ void fetch_l2(const float2 *p, int n, int tid, int nth) {
+  for (int k = 16 * tid; k < n; k += 16 * nth) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p + k));
+}
+// The CTA `ahead` places on in the order of the launch: its PART values, which
+// the plane's other CTAs complete (all of the plane's rows are read by one of
+// them).  Nothing past the launch's last CTA.
+template <int PART>
+__device__ __forceinline__ void fetch_next(const PlaneArgs &a, int tid, int nth) {
+  unsigned b = blockIdx.x + (unsigned)a.ahead, g = blockIdx.y;
+  while (b >= gridDim.x) {
+    b -= gridDim.x;
+    ++g;
+  }
+  if (g < gridDim.y)
+    fetch_l2(reinterpret_cast<const float2 *>(a.g.src[g]) + (long long)b * PART, PART, tid, nth);
+}
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
@@ -112,6 +142,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS
   if constexpr (CS > 1) {
     for (int k = tid; k < NQ; k += NTH) twr[k] = a.wy[r * k];
     if (a.g.src[g] == a.g.dst[g]) cluster_arrive();  // this CTA's rows are read
+    fetch_next<NQ * CX>(a, tid, NTH);
   }
   __syncthreads();
   // 2. x, last stage, in place
@@ -231,7 +262,12 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS
       for (int i = 0; i < R; ++i) d[i * M * P] = v[i];
     }
   }
-  if constexpr (CS > 1) cluster_arrive();
+  if constexpr (CS > 1) {
+    cluster_arrive();
+    fetch_next<NQ * CX>(a, tid, NTH);
+    if (a.g.add[g])  // the plane's addend, read in the last step
+      fetch_l2(reinterpret_cast<const float2 *>(a.g.add[g]) + (long long)blockIdx.x * (NQ * CX), NQ * CX, tid, NTH);
+  }
   __syncthreads();
 
   // 2. y, last stage, and the pre-split of the column pairs, in place
@@ -367,6 +403,18 @@ __global__ void __launch_bounds__(256, 3) k_col_parts(const __grid_constant__ Co
       Dft<R, 1>::run(v);
 #pragma unroll
       for (int i = 0; i < R; ++i) B[swz<CS>(j + i * L::S(0), p)] = v[i];
+    }
+  }
+  {  // a later tile's runs into L2 (see fetch_l2)
+    uint32_t nb = blockIdx.x + a.ahead, ng = g;
+    while (nb >= gridDim.x) {
+      nb -= gridDim.x;
+      ++ng;
+    }
+    if (ng < gridDim.y) {
+      const float2 *next = a.dst[ng] + nb * TXC;
+      for (int k = tid; k < N * CS; k += NTH)
+        asm volatile("prefetch.global.L2 [%0];\n" ::"l"(next + (k / CS) * es + (k % CS) * part));
     }
   }
   __syncthreads();
