@@ -165,7 +165,8 @@ void prof_collect(crava_gpu_ctx *c) {
 //    192x160x384, 48 MB: 1.86 ms on 2 lanes, 1.99 on 3, 1.96 in one launch).
 //  * Larger grids stream from HBM whatever the order: one launch per pass for
 //    all of them has no tails between grids (256x256x512: 4.90 ms per unit
-//    against 5.03 ms on 3 lanes).
+//    against 5.03 ms on 3 lanes, both before the plane passes' fetch into L2,
+//    which also looks ahead from grid to grid of a launch: 4.47).
 constexpr double kOneLaunch = 48e6, kPerLaunch = 24e6, kInL2 = 100e6;
 struct Spread {
   int per, lanes;

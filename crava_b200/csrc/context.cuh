@@ -47,11 +47,10 @@ struct crava_gpu_ctx {
   bool capture = false;
   // synthetic seismic: per-angle spectral filters [ntheta][nzp] (device)
   float2 *synt_H = nullptr;
-  // independent transforms of a unit run on `lanes` streams (1: the
-  // context's stream only), forked from and joined back to it
+  // independent transforms of a unit run on up to `lanes` streams (1: the
+  // context's stream only), forked from and joined back to it; how many a call
+  // uses is the rule at Spread (capi.cu)
   static constexpr int kMaxLanes = 4;
-  // (measured per 256x256x512x5 unit: 6.08 / 5.44 / 5.40 / 5.47 ms with
-  // 1 / 2 / 3 / 4 lanes)
   int lanes = 3;
   cudaStream_t lane_s[kMaxLanes] = {};
   cudaEvent_t lane_fork = nullptr, lane_join[kMaxLanes] = {};

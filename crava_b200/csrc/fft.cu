@@ -5,15 +5,18 @@
 // along y and z, unnormalised, forward sign -) and scale by 1/sqrt(N)
 // (DATA, PARAMETER) or 1 forward / 1/N inverse (COVARIANCE).
 //
-// Three passes, each one read and one write of the grid:
+// The lengths in use have the passes of fft_pass.cuh and plane.cuh, to which
+// the calls below lead.  The passes of this file serve the other lengths and
+// the tuning's explicit choices: three, each one read and one write of the
+// grid:
 //   rows  (x): each CTA transforms ROWS rows of nxp reals; an even nxp is
 //              done as one nxp/2-point complex FFT of the packed row and a
 //              split step (the row's float pairs are read as float2).
 //   cols  (y): each CTA transforms TX adjacent x-columns of one z-plane.
 //   cols  (z): each CTA transforms TX adjacent x-columns of one y-row.
 // Lines live in shared memory and go through the Stockham engine of
-// fft_core.cuh; at the power-of-two lengths 64..512 the register-resident
-// passes of fft_rr.cuh are the default (same arithmetic, fewer shared-memory
+// fft_core.cuh; the power-of-two lengths 64..512 also have the
+// register-resident passes of fft_rr.cuh (same arithmetic, fewer shared-memory
 // round trips).  The scalings are fused into the first (forward) or last
 // (inverse) pass.
 #include <math.h>

@@ -51,17 +51,15 @@ struct FftPlans {
   LinePlan y;        // length nyp
   LinePlan z;        // length nzp
   float2 *xpost = nullptr;  // e^{-2 pi i k/nxp}, k = 0..nxp/2 (even nxp)
-  // column tile of the y and z passes: -1 default, 0 ping-pong pass,
+  // column tile of the y and z passes: -1 default (the built-in pass of
+  // fft_pass.cuh where the length is compiled), 0 ping-pong pass,
   // 1 register-resident pass (lengths 64, 128, 256, 512), 8 or 16 columns
   // per CTA in the in-place pass (lengths with compiled kernels only; other
   // lengths use the generic pass), 2 (z only) the register-resident pass
-  // with TMA tile loads where cols_z_tma_supported.  The default is the
-  // TMA-fed pass where the fused x + y pass is in use and the grid allows
-  // it, else the register-resident pass where it exists, else the in-place
-  // pass.
+  // with TMA tile loads where cols_z_tma_supported.
   int tile_y = -1, tile_z = -1;
-  // x pass of an even nxp: -1 default (register-resident where the half
-  // length is 64..512), 0 the in-place pass, 1 register-resident
+  // x pass: -1 default (the built-in pass where the length is compiled); of
+  // an even nxp 0 the in-place pass, 1 register-resident
   int rows_x = -1;
   // x and y passes in one kernel where the geometry has one: -1 default, 0
   // off, 1 on
@@ -190,8 +188,8 @@ __device__ __forceinline__ unsigned zprior_mask(const ZPrior &z, int t) {
 // its store (where z_prior_supported says the pass has it).
 int fft_cols_z(const FftPlans &p, float2 *grid, int dir, cudaStream_t s, const ZPrior *zp = nullptr);
 // Whether fft_cols_z applies a ZPrior under these plans for every grid of
-// the geometry: the register-resident z pass and its TMA-fed form (lengths
-// 64..512) do, the in-place and generic passes do not.
+// the geometry: the built-in z pass, the register-resident one and its TMA-fed
+// form (lengths 64..512) do, the other in-place and generic passes do not.
 bool z_prior_supported(const FftPlans &p);
 
 // z pass with TMA tile loads (cols_tma.cu; column tile choice 2): lengths

@@ -14,7 +14,8 @@
 // Hermitian in kz (both factors are spectra of real sequences), so two
 // adjacent real traces x = 2p, 2p + 1 are filtered together as one complex
 // line a + i b: the real grid viewed as complex pairs is exactly the
-// complex layout the z column transforms work on.  Traces outside
+// complex layout the z column transforms work on.  The compiled lengths do all
+// of it in one pass (synt_pass.cuh).  Traces outside
 // x < nx, y < ny keep imp, as in the reference.
 #include <math.h>
 

@@ -277,24 +277,24 @@ int crava_gpu_posterior_noalloc(const crava_gpu_params *params,
                                 void *stream, crava_gpu_stats *stats);
 
 /* Launch shapes of a context.  cols_y_tile / cols_z_tile: the y and z
- * column transforms (-1 the built-in choice, 0 the out-of-place pass, 1 the
- * register-resident pass of lengths 64/128/256/512, 8 or 16 columns per CTA
- * in the in-place pass, 2 (z only) the register-resident pass fed by TMA
- * tile loads, where the grid has an even number of lines per z plane;
- * lengths without compiled column kernels ignore it; the built-in z choice
- * is 2 where the fused x + y pass is in use and the grid allows it);
+ * column transforms (-1 the built-in choice: the compiled in-place passes of
+ * all 2, 3, 5, 7-smooth lengths 24..512, several grids per launch; 0 the
+ * out-of-place pass, 1 the register-resident pass of lengths 64/128/256/512, 8
+ * or 16 columns per CTA in the earlier in-place pass, 2 (z only) the
+ * register-resident pass fed by TMA tile loads, where the grid has an even
+ * number of lines per z plane; lengths without compiled column kernels ignore
+ * it);
  * fused: the fused unit kernels (1) or the three passes (0); ms: one unit's
  * measured time (autotune output only); lanes: more than 1 lets the
- * transforms of different grids overlap on that many streams; rows_x: the x
- * pass of an even nxp (-1 built-in, 0 in-place pass, 1 register-resident
- * pass where nxp / 2 is 64..512).  All these choices give the same values
- * bit for bit.  xy_fused: the x and y passes as one thread-block-cluster
- * kernel where the geometry has one (256x256 and 128x128 planes; -1
- * built-in = on where the geometry has it, 0 off, 1 on; alone it is
- * slower than the separate register-resident passes on B200, in the unit
- * beside the TMA-fed z pass faster); it factorises the y transform
- * differently, so it agrees with the separate passes to float rounding,
- * not bit for bit.  kappa_refine (mixed form only, >= 0): an inverted bin whose
+ * transforms of different grids overlap on up to that many streams; rows_x:
+ * the x pass (-1 built-in; of an even nxp 0 in-place pass, 1 register-resident
+ * pass where nxp / 2 is 64..512).  The explicit choices give the same values
+ * bit for bit, the built-in ones agree with them to float rounding.  xy_fused:
+ * the x and y passes as one kernel where the geometry has one (planes with
+ * sides 64 and 128, 256x64, and 256x256 with nzp 64, 128, 256 or 512; -1
+ * built-in = on there unless the tuning names another x or y pass, 0 off, 1
+ * on); it factorises the y transform differently, so it agrees with the
+ * separate passes to float rounding, not bit for bit.  kappa_refine (mixed form only, >= 0): an inverted bin whose
  * FP32 factor has (max L_ii / min L_ii)^2 above it takes one FP64
  * refinement step (0 refines every bin).  solve_shape: the launch shape of
  * the FP64 and mixed solves (-1 built-in: the Woodbury kernel (shape 6)
