@@ -48,7 +48,8 @@ def build(ref: bool | None = None) -> None:
     reference source tree is present (or ref=True)."""
     subprocess.run(["make", "-s", "-C", HERE], check=True)
     if ref is None:
-        ref = os.path.isdir(REF_SRC)
+        # an empty directory is no source tree
+        ref = os.path.isdir(REF_SRC) and bool(os.listdir(REF_SRC))
     if ref:
         if not os.path.isfile(os.path.join(REF_SRC, "libs", "lib", "lib_matr.c")):
             raise FileNotFoundError(f"reference source tree not found at {REF_SRC} "
