@@ -190,16 +190,11 @@ int pass_batch(crava_gpu_ctx *c, const GridBatch &b, int dir, const ZPrior *zp) 
   const double bytes = 2.0 * b.n * (double)c->g.csize * 8.0;
   int rc = CRAVA_GPU_OK;
   const bool fused = use_plane(p);
+  // a split plane's last y step: in the built-in z pass, else in the plane's
+  const bool zparts = fused && p.pass.parts > 1 && use_z_batch(p);
   auto plane = [&] {
     Scope sc(c, dir < 0 ? K_XY_FWD : K_XY_INV, bytes);
-    // a split plane's last y step: in the built-in z pass, else here
-    const bool apart = p.pass.parts > 1 && !use_z_batch(p);
-    for (int i = 0; apart && dir > 0 && i < b.n; ++i)
-      if ((rc = part_radix(p, b.dst[i], dir, c->stream))) return rc;
-    if ((rc = plane_batch(p, b, dir, c->stream))) return rc;
-    for (int i = 0; apart && dir < 0 && i < b.n; ++i)
-      if ((rc = part_radix(p, b.dst[i], dir, c->stream))) return rc;
-    return (int)CRAVA_GPU_OK;
+    return plane_batch(p, b, dir, !zparts, c->stream);
   };
   auto rows = [&] {
     Scope sc(c, dir < 0 ? K_ROWS_FWD : K_ROWS_INV, bytes);
@@ -217,7 +212,7 @@ int pass_batch(crava_gpu_ctx *c, const GridBatch &b, int dir, const ZPrior *zp) 
   };
   auto z = [&] {
     Scope sc(c, dir < 0 ? K_COLS_Z_FWD : K_COLS_Z_INV, bytes);
-    if (use_z_batch(p)) return z_batch(p, b, dir, fused && p.pass.parts > 1, zp, c->stream);
+    if (use_z_batch(p)) return z_batch(p, b, dir, zparts, zp, c->stream);
     for (int i = 0; i < b.n; ++i)
       if ((rc = fft_cols_z(p, reinterpret_cast<float2 *>(b.dst[i]), dir, c->stream, zp ? zp + i : nullptr))) return rc;
     return (int)CRAVA_GPU_OK;
@@ -647,10 +642,7 @@ int crava_gpu_fft_xy(crava_gpu_ctx *c, float *grid, int dir, int type, int nzp_f
   if (use_plane(c->plans)) {
     GridBatch b;
     b.push(grid, grid, scale);
-    const bool parts = c->plans.pass.parts > 1;
-    if (dir > 0 && parts && (rc = part_radix(c->plans, grid, dir, c->stream))) return rc;
-    if ((rc = plane_batch(c->plans, b, dir, c->stream))) return rc;
-    return dir < 0 && parts ? part_radix(c->plans, grid, dir, c->stream) : (int)CRAVA_GPU_OK;
+    return plane_batch(c->plans, b, dir, true, c->stream);
   }
   if (dir < 0) {
     if ((rc = fft_rows(c->plans, grid, -1, scale, c->stream))) return rc;

@@ -76,11 +76,10 @@ void pass_plan_destroy(PassPlan *p);
 int rows_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);
 int y_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);
 int z_batch(const FftPlans &p, const GridBatch &b, int dir, bool parts, const ZPrior *zp, cudaStream_t s);
-// The fused x + y pass; where it splits a plane (p.pass.parts 2) without the
-// last y step over the parts, which z_batch (parts) or part_radix does.
+// The fused x + y pass; where it splits a plane (p.pass.parts 2) with the last y
+// step over the parts (whole), or without it, where z_batch (parts) does it.
 int plane_parts(const Geom &g);
-int plane_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s);
-int part_radix(const FftPlans &p, float *grid, int dir, cudaStream_t s);
+int plane_batch(const FftPlans &p, const GridBatch &b, int dir, bool whole, cudaStream_t s);
 // Which passes of these plans they do: where the length is compiled and the
 // tuning names no other.
 inline bool use_rows_batch(const FftPlans &p) { return p.rows_x == -1 && p.pass.xf; }

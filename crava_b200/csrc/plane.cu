@@ -12,11 +12,11 @@ int sm_count(int *n) {
   return CRAVA_GPU_OK;
 }
 
-template <int NX, int NY, int CS>
+template <int NX, int NY, int CS, bool WHOLE = false>
 int launch_plane(PlaneArgs a, int dir, int nplanes, int ngrids, cudaStream_t s) {
   using C = PlaneCfg<NX, NY, CS>;
-  const void *fn = dir < 0 ? (const void *)k_plane_fwd<NX, NY, CS> : (const void *)k_plane_inv<NX, NY, CS>;
-  const size_t smem = C::smem(dir);
+  const void *fn = dir < 0 ? (const void *)k_plane_fwd<NX, NY, CS, WHOLE> : (const void *)k_plane_inv<NX, NY, CS, WHOLE>;
+  const size_t smem = WHOLE ? C::smem_whole(dir) : C::smem(dir);
   int rc = func_smem(fn, smem);
   if (rc) return rc;
   a.ahead = 0;
@@ -33,8 +33,8 @@ int launch_plane(PlaneArgs a, int dir, int nplanes, int ngrids, cudaStream_t s) 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = CS > 1 ? 1 : 0;
-  if (dir < 0) CRAVA_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_plane_fwd<NX, NY, CS>, a));
-  else CRAVA_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_plane_inv<NX, NY, CS>, a));
+  if (dir < 0) CRAVA_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_plane_fwd<NX, NY, CS, WHOLE>, a));
+  else CRAVA_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_plane_inv<NX, NY, CS, WHOLE>, a));
   note_launch();
   return CRAVA_GPU_OK;
 }
@@ -54,18 +54,6 @@ int launch_parts(ColPassArgs a, int ngrids, int dir, cudaStream_t s) {
   return CRAVA_GPU_OK;
 }
 
-// The radix-2 step over the parts as a pass of its own (fft_xy).
-template <int DIR>
-__global__ void __launch_bounds__(256) k_part_radix2(float2 *grid, long long part, long long plane) {
-  float2 *g = grid + (long long)blockIdx.y * plane;
-  for (long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x; f < part; f += (long long)gridDim.x * blockDim.x) {
-    float2 v[2] = {g[f], g[f + part]};
-    Dft<2, DIR>::run(v);
-    g[f] = v[0];
-    g[f + part] = v[1];
-  }
-}
-
 }  // namespace
 
 // CTAs per plane; 0: the geometry takes the separate passes.  One where a plane
@@ -79,7 +67,7 @@ int plane_parts(const Geom &g) {
 
 bool plane_xy_supported(const Geom &g) { return plane_parts(g) > 0; }
 
-int plane_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) {
+int plane_batch(const FftPlans &p, const GridBatch &b, int dir, bool whole, cudaStream_t s) {
   const Geom &g = p.g;
   PlaneArgs a;
   for (int i = 0; i < b.n; ++i) {
@@ -96,8 +84,10 @@ int plane_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) 
   if (g.nxp == NX && g.nyp == NY) return launch_plane<NX, NY, CS>(a, dir, g.nzp, b.n, s);
   CRAVA_PLANE(64, 64, 1) CRAVA_PLANE(64, 128, 1)
   CRAVA_PLANE(128, 64, 1) CRAVA_PLANE(128, 128, 1)
-  CRAVA_PLANE(256, 64, 1) CRAVA_PLANE(256, 256, 2)
+  CRAVA_PLANE(256, 64, 1)
 #undef CRAVA_PLANE
+  if (g.nxp == 256 && g.nyp == 256)
+    return whole ? launch_plane<256, 256, 2, true>(a, dir, g.nzp, b.n, s) : launch_plane<256, 256, 2>(a, dir, g.nzp, b.n, s);
   return CRAVA_GPU_ERR_ARG;
 }
 
@@ -109,17 +99,6 @@ int z_parts_launch(const ColPassArgs &a, int n, int ngrids, int dir, cudaStream_
     case 512: return launch_parts<512, 2>(a, ngrids, dir, s);
     default: return CRAVA_GPU_ERR_ARG;
   }
-}
-
-int part_radix(const FftPlans &p, float *real, int dir, cudaStream_t s) {
-  const Geom &g = p.g;
-  float2 *grid = reinterpret_cast<float2 *>(real);
-  const long long plane = (long long)g.cnxp * g.nyp;
-  const dim3 grd(64, (unsigned)g.nzp);
-  if (dir < 0) k_part_radix2<-1><<<grd, 256, 0, s>>>(grid, plane / 2, plane);
-  else k_part_radix2<1><<<grd, 256, 0, s>>>(grid, plane / 2, plane);
-  CRAVA_LAUNCH_CHECK();
-  return CRAVA_GPU_OK;
 }
 
 }  // namespace crava

@@ -15,6 +15,18 @@
 // CTA's input rows: the two form a cluster, each arrives at its barrier when its
 // loads are done and waits there before its first store.
 //
+// Where no such z pass follows (the x and y passes of a slab, or another z pass
+// by the tuning) the kernel does the radix-2 step itself (WHOLE), with the same
+// values.  Forward each CTA takes the rows of half of the k1 and pushes its
+// brackets of the other half into the partner's shared memory, in the order of
+// the columns (66 KB more, 215 in all); inverse each CTA reads both rows k1 and
+// k1 + NQ of the pair and forms its own part's, the second reading coming from
+// L2 as the two run at once.  One slab of 256x256x512: 116 / 97 us forward /
+// inverse, of 64 planes 20.6 / 17.5 (the earlier cluster of four CTAs 121 / 110 and
+// 24.7 / 20.6; the parts kernel and a radix-2 pass after it 141 / 140 and 24.1 /
+// 22.9).  Forward, the partner's brackets pulled from the slots they lie in,
+// scattered over the banks, took 131 us, handed over through L2 123.
+//
 // The split of the packed x line into the half spectrum pairs column k with
 // nh - k; the first y stage (forward) or the last one (inverse) takes the two
 // columns of a pair together and does it in registers.
@@ -55,6 +67,8 @@ struct PlaneCfg {
   static constexpr size_t smem(int dir) {
     return sizeof(float2) * ((size_t)NQ * (dir < 0 ? PF : PI) + (CS > 1 ? NQ : 0));
   }
+  // the forward kernel that completes y receives half of the partner's rows
+  static constexpr size_t smem_whole(int dir) { return smem(dir) + (dir < 0 ? sizeof(float2) * (size_t)(NQ / 2) * CX : 0); }
   static constexpr int kCtas = 224 * 1024 / (int)(smem(PF > PI ? -1 : 1) + 1024) >= 3 ? 3
                                : 224 * 1024 / (int)(smem(PF > PI ? -1 : 1) + 1024) >= 2 ? 2 : 1;
   static constexpr int NTH = kCtas == 3 ? 256 : kCtas == 2 ? 512 : 1024;
@@ -103,7 +117,16 @@ __device__ __forceinline__ void fetch_next(const PlaneArgs &a, int tid, int nth)
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
 
-template <int NX, int NY, int CS>
+__device__ __forceinline__ uint32_t cluster_addr(const void *smem, uint32_t rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(smem)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, float2 v) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
+}
+
+template <int NX, int NY, int CS, bool WHOLE>
 __global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS>::kMinB)
     k_plane_fwd(const __grid_constant__ PlaneArgs a) {
   using C = PlaneCfg<NX, NY, CS>;
@@ -113,6 +136,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS
   constexpr LY ly{};
   constexpr int NTH = C::NTH, NQ = C::NQ, NH = C::NH, CX = C::CX, NP = C::NP, P = C::PF, SPARE = LX::R(0) * LX::S(0);
   static_assert(LX::nst() == 2 && LY::nst() == 2, "two-stage lines");
+  static_assert(!WHOLE || CS == 2, "the radix-2 step over two parts");
   extern __shared__ float4 sm4[];
   float2 *A = reinterpret_cast<float2 *>(sm4), *twr = A + NQ * P;
   const int tid = threadIdx.x;
@@ -141,7 +165,7 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS
   }
   if constexpr (CS > 1) {
     for (int k = tid; k < NQ; k += NTH) twr[k] = a.wy[r * k];
-    if (a.g.src[g] == a.g.dst[g]) cluster_arrive();  // this CTA's rows are read
+    if (WHOLE || a.g.src[g] == a.g.dst[g]) cluster_arrive();  // this CTA's rows are read
     fetch_next<NQ * CX>(a, tid, NTH);
   }
   __syncthreads();
@@ -197,29 +221,87 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS
   __syncthreads();
 
   // 4. y, last stage: shared memory -> registers -> HBM
-  if constexpr (CS > 1) if (a.g.src[g] == a.g.dst[g]) cluster_wait();  // every CTA of the plane has read its rows
-  {
-    constexpr int R = LY::R(1), M = LY::M(1), S = LY::S(1);
+  constexpr int R = LY::R(1), M = LY::M(1), S = LY::S(1);
+  auto last = [&](int t, float2 *v) {  // the brackets of rows j + i M, column k; their first slot
+    const int j = t / CX, k = t % CX;
+    float2 *o = A + line_slot(ly, 1, j) * P + (k == NH ? SPARE : line_out(lx, k));
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = o[i * S * P];
+    line_twiddle<R, -1>(ly, 1, j, v, a.twy);
+    Dft<R, -1>::run(v);
+    if constexpr (CS > 1) {
+#pragma unroll
+      for (int i = 0; i < R; ++i) v[i] = cmul(v[i], twr[j + i * M]);
+    }
+    return o;
+  };
+  if constexpr (!WHOLE) {
+    if constexpr (CS > 1) if (a.g.src[g] == a.g.dst[g]) cluster_wait();  // every CTA of the plane has read its rows
 #pragma unroll 1
     for (int t = tid; t < CX * M; t += NTH) {
-      const int j = t / CX, k = t % CX;
-      const float2 *o = A + line_slot(ly, 1, j) * P + (k == NH ? SPARE : line_out(lx, k));
       float2 v[R];
+      last(t, v);
+      float2 *d = dst + (t / CX) * CX + t % CX;
 #pragma unroll
-      for (int i = 0; i < R; ++i) v[i] = o[i * S * P];
-      line_twiddle<R, -1>(ly, 1, j, v, a.twy);
-      Dft<R, -1>::run(v);
-      float2 *d = dst + j * CX + k;
+      for (int i = 0; i < R; ++i) d[i * M * CX] = v[i];
+    }
+  } else {
+    // and the radix-2 step: this CTA takes the rows of half of the i.  A
+    // butterfly keeps that half (in registers; those of the columns past a whole
+    // round, a few, in their slots) and pushes the other into the partner's
+    // shared memory, in the order of the columns
+    constexpr int H = R / 2;
+    static_assert(NTH < CX * M && CX * M <= 2 * NTH, "one butterfly per thread and a remainder");
+    const int i0 = r * H;  // first i of this CTA's rows
+    float2 *B = twr + NQ;  // [H][CX M]: the partner's brackets of this CTA's rows
+    const uint32_t to = cluster_addr(B, r ^ 1);
+    float2 *out = reinterpret_cast<float2 *>(a.g.dst[g]) + (long long)plane * CX * NY;
+    const int t1 = tid + NTH;
+    const bool rest = t1 < CX * M;
+    cluster_wait();  // the partner runs, and has read its rows
+    auto push = [&](int t, const float2 *v) {
 #pragma unroll
-      for (int i = 0; i < R; ++i) {
-        if constexpr (CS > 1) d[i * M * CX] = cmul(v[i], twr[j + i * M]);
-        else d[i * M * CX] = v[i];
+      for (int i = 0; i < H; ++i) cluster_store(to + (uint32_t)sizeof(float2) * (i * CX * M + t), r == 0 ? v[i + H] : v[i]);
+    };
+    float2 keep[H];
+    float2 *slot = nullptr;
+    if (rest) {
+      float2 v[R];
+      slot = last(t1, v) + i0 * S * P;
+      push(t1, v);
+#pragma unroll
+      for (int i = 0; i < H; ++i) slot[i * S * P] = r == 0 ? v[i] : v[i + H];
+    }
+    {
+      float2 v[R];
+      last(tid, v);
+      push(tid, v);
+#pragma unroll
+      for (int i = 0; i < H; ++i) keep[i] = r == 0 ? v[i] : v[i + H];
+    }
+    cluster_arrive();  // this CTA's pushes are done
+    cluster_wait();
+    auto finish = [&](int t) {
+      float2 *d = out + (t / CX + i0 * M) * CX + t % CX;
+#pragma unroll
+      for (int i = 0; i < H; ++i) {
+        const float2 his = B[i * CX * M + t];
+        float2 v[2] = {r == 0 ? keep[i] : his, r == 0 ? his : keep[i]};
+        Dft<2, -1>::run(v);
+        d[i * M * CX] = v[0];
+        d[(i * M + NQ) * CX] = v[1];
       }
+    };
+    finish(tid);
+    if (rest) {
+#pragma unroll
+      for (int i = 0; i < H; ++i) keep[i] = slot[i * S * P];
+      finish(t1);
     }
   }
 }
 
-template <int NX, int NY, int CS>
+template <int NX, int NY, int CS, bool WHOLE>
 __global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS>::kMinB)
     k_plane_inv(const __grid_constant__ PlaneArgs a) {
   using C = PlaneCfg<NX, NY, CS>;
@@ -232,7 +314,9 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS
   float2 *A = reinterpret_cast<float2 *>(sm4), *twr = A + NQ * P;
   const int tid = threadIdx.x;
   const int plane = blockIdx.x / CS, r = blockIdx.x % CS, g = blockIdx.y;
-  const float2 *src = reinterpret_cast<const float2 *>(a.g.src[g]) + (long long)plane * CX * NY + (long long)r * NQ * CX;
+  static_assert(!WHOLE || CS == 2, "the radix-2 step over two parts");
+  const float2 *src = reinterpret_cast<const float2 *>(a.g.src[g]) + (long long)plane * CX * NY +
+                      (WHOLE ? 0 : (long long)r * NQ * CX);
   const long long off = (long long)plane * CX * NY + r * CX;
   float2 *dst = reinterpret_cast<float2 *>(a.g.dst[g]) + off;
   const float2 *add = a.g.add[g] ? reinterpret_cast<const float2 *>(a.g.add[g]) + off : nullptr;
@@ -251,7 +335,13 @@ __global__ void __launch_bounds__(PlaneCfg<NX, NY, CS>::NTH, PlaneCfg<NX, NY, CS
       const float2 *o = src + j * CX + k;
       float2 v[R];
 #pragma unroll
-      for (int i = 0; i < R; ++i) v[i] = o[i * M * CX];
+      for (int i = 0; i < R; ++i) {
+        v[i] = o[i * M * CX];
+        if constexpr (WHOLE) {  // the radix-2 step over the two parts: this part's output
+          const float2 w = o[(i * M + NQ) * CX];
+          v[i] = r == 0 ? cadd(v[i], w) : csub(v[i], w);
+        }
+      }
       if constexpr (CS > 1) {
 #pragma unroll
         for (int i = 0; i < R; ++i) v[i] = cmul(v[i], twr[j + i * M]);

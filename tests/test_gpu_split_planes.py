@@ -1,0 +1,54 @@
+"""256x256 planes, which the fused x + y pass splits over two CTAs: the last y
+step over the two parts is the z pass's first butterfly where that z pass
+follows, and the plane kernel's own where it does not (the x and y passes of a
+slab, a z pass that the tuning names).  Both are one pass over the plane and
+give the same values."""
+import numpy as np
+import pytest
+import torch
+
+from crava_b200 import api, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _context(nx, ny, nz):
+    return api.Context(synth.Case(
+        nxp=nx, nyp=ny, nzp=nz, angles_deg=[10.0], dt=4.0, low_cut=5.0, high_cut=55.0, wnc=0.1, nz=nz, lz=nz * 4.0,
+        min_rel_thick=1.0, wavelet=synth.ricker_fft_order(nz, 4.0)[None], A=synth.aki_richards_pp([10.0]),
+        theta_cov=np.eye(1), var0=synth.prior_var0(), mu=[], data=[], cov=[], err_corr=None))
+
+
+def _grid(nx, ny, nz, seed=1):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn((nz, ny, 2 * (nx // 2 + 1)), device="cuda", generator=gen)
+
+
+def _launches(f):
+    n = api.launch_count()
+    f()
+    torch.cuda.synchronize()
+    return api.launch_count() - n
+
+
+@pytest.mark.parametrize("nz", [64, 128])
+def test_x_and_y_of_a_slab_in_one_pass(nz):
+    ctx = _context(256, 256, nz)
+    g = _grid(256, 256, nz)
+    assert _launches(lambda: ctx.fft_xy(g, -1, api.DATA)) == 1
+    assert _launches(lambda: ctx.fft_xy(g, 1, api.DATA)) == 1
+
+
+@pytest.mark.parametrize("tile_z", [16, 1, 2])
+def test_named_z_pass_follows_the_whole_plane_pass(tile_z):
+    """Two passes, and the values of the z pass that completes y itself."""
+    ctx = _context(256, 256, 64)
+    a, b = _grid(256, 256, 64), _grid(256, 256, 64)
+    ctx.fft_r2c(a, api.PARAMETER)
+    ctx.set_tuning(-1, tile_z, 0, 3, -1, None, 1)
+    assert _launches(lambda: ctx.fft_r2c(b, api.PARAMETER)) == 2
+    assert torch.equal(a, b)
+    assert _launches(lambda: ctx.fft_c2r(b, api.PARAMETER)) == 2
+    ctx.set_tuning(-1, -1, 0, 3, -1, None, -1)
+    ctx.fft_c2r(a, api.PARAMETER)
+    assert torch.equal(a, b)
