@@ -190,8 +190,8 @@ int pass_batch(crava_gpu_ctx *c, const GridBatch &b, int dir, const ZPrior *zp) 
   const double bytes = 2.0 * b.n * (double)c->g.csize * 8.0;
   int rc = CRAVA_GPU_OK;
   const bool fused = use_plane(p);
-  // a split plane's last y step: in the built-in z pass, else in the plane's
-  const bool zparts = fused && p.pass.parts > 1 && use_z_batch(p);
+  // a split plane's last y step: in the z pass that does it, else in the plane's
+  const bool zparts = fused && use_z_parts(p);
   auto plane = [&] {
     Scope sc(c, dir < 0 ? K_XY_FWD : K_XY_INV, bytes);
     return plane_batch(p, b, dir, !zparts, c->stream);

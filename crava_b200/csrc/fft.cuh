@@ -79,16 +79,23 @@ int z_batch(const FftPlans &p, const GridBatch &b, int dir, bool parts, const ZP
 // The fused x + y pass; where it splits a plane (p.pass.parts 2) with the last y
 // step over the parts (whole), or without it, where z_batch (parts) does it.
 int plane_parts(const Geom &g);
+inline bool z_parts_length(int nzp) { return nzp == 64 || nzp == 128 || nzp == 256 || nzp == 512; }
 int plane_batch(const FftPlans &p, const GridBatch &b, int dir, bool whole, cudaStream_t s);
 // Which passes of these plans they do: where the length is compiled and the
 // tuning names no other.
 inline bool use_rows_batch(const FftPlans &p) { return p.rows_x == -1 && p.pass.xf; }
 inline bool use_y_batch(const FftPlans &p) { return p.tile_y == -1 && p.pass.y; }
 inline bool use_z_batch(const FftPlans &p) { return p.tile_z == -1 && p.pass.z; }
-// The fused x + y pass: where the geometry has it, unless the tuning turns it
-// off or names one of the separate x and y passes (xy_fused 1: on all the same).
+// Whether that z pass is the one that completes the y of planes split in two.
+inline bool use_z_parts(const FftPlans &p) { return p.pass.parts > 1 && use_z_batch(p) && z_parts_length(p.g.nzp); }
+// The fused x + y pass, where the plane has it: by the tuning (xy_fused 1), else
+// unless the tuning turns it off or names one of the separate x and y passes; a
+// split plane then also wants the z pass that completes it (without it 116 / 97
+// us per 256x256x512 grid, forward / inverse, against 43 + 44 / 46 + 51 for the
+// separate passes).
 inline bool use_plane(const FftPlans &p) {
-  return p.pass.parts && (p.plane_xy == 1 || (p.plane_xy == -1 && p.tile_y == -1 && p.rows_x == -1));
+  const bool built_in = p.pass.parts == 1 || z_parts_length(p.g.nzp);
+  return p.pass.parts && (p.plane_xy == 1 || (p.plane_xy == -1 && p.tile_y == -1 && p.rows_x == -1 && built_in));
 }
 
 // Whether length n has compiled column kernels (tile choices 0, 8, 16).

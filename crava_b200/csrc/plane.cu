@@ -56,13 +56,12 @@ int launch_parts(ColPassArgs a, int ngrids, int dir, cudaStream_t s) {
 
 }  // namespace
 
-// CTAs per plane; 0: the geometry takes the separate passes.  One where a plane
-// fits 75 KB; two at 256x256 where the z line has the pass that completes y.
+// CTAs per plane; 0: the plane has the separate passes alone.  One where a plane
+// fits a CTA with others on the SM, two at 256x256.
 int plane_parts(const Geom &g) {
   const bool px = g.nxp == 64 || g.nxp == 128, py = g.nyp == 64 || g.nyp == 128;
   if ((px && py) || (g.nxp == 256 && g.nyp == 64)) return 1;
-  const bool z = g.nzp == 64 || g.nzp == 128 || g.nzp == 256 || g.nzp == 512;
-  return g.nxp == 256 && g.nyp == 256 && z ? 2 : 0;
+  return g.nxp == 256 && g.nyp == 256 ? 2 : 0;
 }
 
 bool plane_xy_supported(const Geom &g) { return plane_parts(g) > 0; }
@@ -92,7 +91,7 @@ int plane_batch(const FftPlans &p, const GridBatch &b, int dir, bool whole, cuda
 }
 
 int z_parts_launch(const ColPassArgs &a, int n, int ngrids, int dir, cudaStream_t s) {
-  switch (n) {
+  switch (n) {  // z_parts_length
     case 64: return launch_parts<64, 2>(a, ngrids, dir, s);
     case 128: return launch_parts<128, 2>(a, ngrids, dir, s);
     case 256: return launch_parts<256, 2>(a, ngrids, dir, s);

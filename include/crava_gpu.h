@@ -290,10 +290,9 @@ int crava_gpu_posterior_noalloc(const crava_gpu_params *params,
  * the x pass (-1 built-in; of an even nxp 0 in-place pass, 1 register-resident
  * pass where nxp / 2 is 64..512).  The explicit choices give the same values
  * bit for bit, the built-in ones agree with them to float rounding.  xy_fused:
- * the x and y passes as one kernel where the geometry has one (planes with
- * sides 64 and 128, 256x64, and 256x256 with nzp 64, 128, 256 or 512; -1
- * built-in = on there unless the tuning names another x or y pass, 0 off, 1
- * on); it factorises the y transform differently, so it agrees with the
+ * the x and y passes as one kernel where the plane has one (sides 64 and
+ * 128, 256x64, 256x256; 0 off, 1 on, -1 built-in = on there unless the tuning
+ * names another x or y pass, at 256x256 for nzp 64, 128, 256 and 512); it factorises the y transform differently, so it agrees with the
  * separate passes to float rounding, not bit for bit.  kappa_refine (mixed form only, >= 0): an inverted bin whose
  * FP32 factor has (max L_ii / min L_ii)^2 above it takes one FP64
  * refinement step (0 refines every bin).  solve_shape: the launch shape of

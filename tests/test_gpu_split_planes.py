@@ -52,3 +52,21 @@ def test_named_z_pass_follows_the_whole_plane_pass(tile_z):
     ctx.set_tuning(-1, -1, 0, 3, -1, None, -1)
     ctx.fft_c2r(a, api.PARAMETER)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("nz,tile_z", [(16, -1), (60, -1), (60, 2), (96, 8)])
+def test_fused_pass_on_at_any_depth(nz, tile_z):
+    """xy_fused = 1 is one pass over the planes whatever the z length, 0 two;
+    a float32 transform of N points is within eps log2(N) / 2, eps = 2^-24."""
+    ctx = _context(256, 256, nz)
+    g = _grid(256, 256, nz)
+    ref = torch.fft.rfftn(g[..., :256].double()) / np.sqrt(256 * 256 * nz)
+    for xy, passes in ((1, 2), (0, 3)):
+        ctx.set_tuning(-1, tile_z, 0, 3, -1, None, xy)
+        t = g.clone()
+        assert _launches(lambda: ctx.fft_r2c(t, api.PARAMETER)) == passes
+        spec = torch.view_as_complex(t.view(nz, 256, 129, 2)).to(ref.dtype)
+        assert float((spec - ref).norm() / ref.norm()) < 7.6e-7
+        assert _launches(lambda: ctx.fft_c2r(t, api.PARAMETER)) == passes
+        assert float((t - g)[..., :256].norm() / g[..., :256].norm()) < 2 * 7.6e-7
+        assert float(t[..., 256:].abs().max()) == 0.0
