@@ -639,7 +639,9 @@ int crava_gpu_fft_xy(crava_gpu_ctx *c, float *grid, int dir, int type, int nzp_f
   const Geom full = Geom::make(c->g.nxp, c->g.nyp, nzp_full);
   const float scale = dir < 0 ? forward_scale(full, type) : inverse_scale(full, type);
   int rc;
-  if (use_plane(c->plans)) {
+  // the x + y pass of the whole grid's transforms, whose values it then has
+  // whatever the slab's depth
+  if (use_plane(c->plans, nzp_full)) {
     GridBatch b;
     b.push(grid, grid, scale);
     return plane_batch(c->plans, b, dir, true, c->stream);

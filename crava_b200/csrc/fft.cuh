@@ -92,11 +92,12 @@ inline bool use_z_parts(const FftPlans &p) { return p.pass.parts > 1 && use_z_ba
 // unless the tuning turns it off or names one of the separate x and y passes; a
 // split plane then also wants the z pass that completes it (without it 116 / 97
 // us per 256x256x512 grid, forward / inverse, against 43 + 44 / 46 + 51 for the
-// separate passes).
-inline bool use_plane(const FftPlans &p) {
-  const bool built_in = p.pass.parts == 1 || z_parts_length(p.g.nzp);
+// separate passes).  nzp: the planes of the whole grid, where p is a slab's.
+inline bool use_plane(const FftPlans &p, int nzp) {
+  const bool built_in = p.pass.parts == 1 || z_parts_length(nzp);
   return p.pass.parts && (p.plane_xy == 1 || (p.plane_xy == -1 && p.tile_y == -1 && p.rows_x == -1 && built_in));
 }
+inline bool use_plane(const FftPlans &p) { return use_plane(p, p.g.nzp); }
 
 // Whether length n has compiled column kernels (tile choices 0, 8, 16).
 bool cols_tunable(int n);

@@ -130,8 +130,9 @@ int crava_gpu_fft_c2r(crava_gpu_ctx *ctx, float *grid, int grid_type);
  * geometry (a slab: the context's nzp planes of a grid of nzp_full), the
  * real <-> half-complex x transform scaled as fftInPlace / invFFTInPlace
  * scale the whole grid of grid_type; crava_gpu_fft_z runs the unscaled
- * complex z pass over every column.  On one GPU (nzp_full = nzp) they
- * equal crava_gpu_fft_r2c / _c2r bit for bit. */
+ * complex z pass over every column.  Slab by slab and shard by shard they
+ * equal crava_gpu_fft_r2c / _c2r of the whole grid bit for bit, the contexts
+ * tuned alike. */
 int crava_gpu_fft_xy(crava_gpu_ctx *ctx, float *grid, int dir, int grid_type, int nzp_full);
 int crava_gpu_fft_z(crava_gpu_ctx *ctx, float *grid, int dir);
 

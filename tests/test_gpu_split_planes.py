@@ -70,3 +70,32 @@ def test_fused_pass_on_at_any_depth(nz, tile_z):
         assert _launches(lambda: ctx.fft_c2r(t, api.PARAMETER)) == passes
         assert float((t - g)[..., :256].norm() / g[..., :256].norm()) < 2 * 7.6e-7
         assert float(t[..., 256:].abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("shape,slabs", [
+    ((256, 256, 128), (32, 96)),   # the whole grid has the two-part planes, a slab's depth alone would not
+    ((256, 256, 192), (64, 128)),  # the other way round
+    ((128, 128, 54), (24, 30)),
+    ((64, 48, 50), (25, 25)),
+])
+def test_slabs_equal_the_whole_transform(shape, slabs):
+    """The x and y passes slab by slab and the z pass are the 3-D transform of
+    the whole grid bit for bit, forward and inverse."""
+    nx, ny, nz = shape
+    whole = _context(nx, ny, nz)
+    parts, z0 = [], 0
+    for n in slabs:
+        parts.append((_context(nx, ny, n), slice(z0, z0 + n)))
+        z0 += n
+    a = _grid(nx, ny, nz)
+    b = a.clone()
+    whole.fft_r2c(a, api.PARAMETER)
+    for ctx, s in parts:
+        ctx.fft_xy(b[s], -1, api.PARAMETER, nz)
+    whole.fft_z(b, -1)
+    assert torch.equal(a, b)
+    whole.fft_c2r(a, api.PARAMETER)
+    whole.fft_z(b, 1)
+    for ctx, s in parts:
+        ctx.fft_xy(b[s], 1, api.PARAMETER, nz)
+    assert torch.equal(a, b)
