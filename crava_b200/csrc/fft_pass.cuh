@@ -4,8 +4,9 @@
 // Rows (x): a CTA transforms kB rows of nxp reals.  Even nxp: the packed
 // nxp / 2-point complex line; the split into the half spectrum (forward) or
 // out of it (inverse) pairs position k with nh - k, one thread doing both.
-// Odd nxp: two rows at a time as real and imaginary part of one nxp-point
-// line.
+// Odd nxp: two rows of a plane at a time as real and imaginary part of one
+// nxp-point line (the last of an odd nyp alone), so that a plane's values do not
+// hang on its neighbours', nor on which planes are in the grid.
 // Columns (y and z): a CTA transforms 16 adjacent lines, 128 bytes of every
 // row it touches; lanes run along the lines, so a shared-memory row is one
 // 128-byte access whatever the stage and a warp reads two twiddles.
@@ -34,7 +35,9 @@ struct PassGrids {
 // ------------------------------------------------------------------ rows
 struct RowPassArgs {
   PassGrids g;
-  long long nrows;    // nyp nzp
+  uint32_t nlines;    // rows, nyp nzp (odd nxp: pairs, ceil(nyp / 2) nzp)
+  uint32_t odd;       // nyp mod 2
+  FastDiv fpairs;     // ceil(nyp / 2)
   const float2 *tw;   // stage tables of the direction's line
   const float2 *post; // W_nxp^k, k <= nxp / 2 (even nxp)
 };
@@ -248,10 +251,21 @@ __device__ __forceinline__ void rows_inv_even(const float *src, float *dst, cons
   }
 }
 
-// Odd nxp: line q of a tile holds rows 2 q and 2 q + 1.
+// Odd nxp: the first row of pair l, and whether the pair has a second one.
+struct RowPair {
+  uint32_t row;
+  bool two;
+};
+__device__ __forceinline__ RowPair row_pair(const RowPassArgs &a, uint32_t l) {
+  if (!a.odd) return RowPair{2 * l, true};
+  const uint32_t plane = fdiv(l, a.fpairs);
+  return RowPair{2 * l - plane, l - plane * a.fpairs.d + 1 != a.fpairs.d};
+}
+
+// Odd nxp: the pairs line0 .. line0 + B of rows.
 template <int NX, int NTH>
-__device__ __forceinline__ void rows_fwd_odd(const float *src, float *dst, long long row0, int nrows, float scale,
-                                             const float2 *tw, float2 *A, int tid) {
+__device__ __forceinline__ void rows_fwd_odd(const RowPassArgs &a, const float *src, float *dst, uint32_t line0,
+                                             int nlines, float scale, const float2 *tw, float2 *A, int tid) {
   using C = RowCfg<NX>;
   using L = typename C::F;
   constexpr L l{};
@@ -261,8 +275,9 @@ __device__ __forceinline__ void rows_fwd_odd(const float *src, float *dst, long 
 #pragma unroll 1
     for (int t = tid; t < B * M; t += NTH) {
       const int q = t / M, j = t % M;
-      const float *ra = src + (row0 + (2 * q < nrows ? 2 * q : 0)) * RX + j;
-      const bool two = 2 * q + 1 < nrows;
+      const RowPair pr = row_pair(a, line0 + (q < nlines ? q : 0));
+      const float *ra = src + (size_t)pr.row * RX + j;
+      const bool two = pr.two;
       const float *rb = two ? ra + RX : ra;
       float2 v[R];
 #pragma unroll
@@ -285,18 +300,20 @@ __device__ __forceinline__ void rows_fwd_odd(const float *src, float *dst, long 
 #pragma unroll 1
   for (int t = tid; t < B * CX; t += NTH) {
     const int q = t / CX, k = t % CX;
-    if (2 * q >= nrows) continue;
+    if (q >= nlines) continue;
+    const RowPair pr = row_pair(a, line0 + q);
     const float2 *z = A + q * P;
     const float2 zk = z[line_out(l, k)], zm = k == 0 ? zk : z[line_out(l, N - k)];
-    float2 *o = reinterpret_cast<float2 *>(dst) + (row0 + 2 * q) * CX + k;
+    float2 *o = reinterpret_cast<float2 *>(dst) + (size_t)pr.row * CX + k;
     o[0] = make_float2(h * (zk.x + zm.x), h * (zk.y - zm.y));
-    if (2 * q + 1 < nrows) o[CX] = make_float2(h * (zk.y + zm.y), h * (zm.x - zk.x));
+    if (pr.two) o[CX] = make_float2(h * (zk.y + zm.y), h * (zm.x - zk.x));
   }
 }
 
 template <int NX, int NTH>
-__device__ __forceinline__ void rows_inv_odd(const float *src, float *dst, const float *add, long long row0, int nrows,
-                                             float scale, const float2 *tw, float2 *A, int tid) {
+__device__ __forceinline__ void rows_inv_odd(const RowPassArgs &a, const float *src, float *dst, const float *add,
+                                             uint32_t line0, int nlines, float scale, const float2 *tw, float2 *A,
+                                             int tid) {
   using C = RowCfg<NX>;
   using L = typename C::I;
   constexpr L l{};
@@ -306,8 +323,9 @@ __device__ __forceinline__ void rows_inv_odd(const float *src, float *dst, const
 #pragma unroll 1
   for (int t = tid; t < B * CX; t += NTH) {
     const int q = t / CX, k = t % CX;
-    const float2 *X = reinterpret_cast<const float2 *>(src) + (row0 + (2 * q < nrows ? 2 * q : 0)) * CX + k;
-    const float2 xa = X[0], xb = 2 * q + 1 < nrows ? X[CX] : make_float2(0.f, 0.f);
+    const RowPair pr = row_pair(a, line0 + (q < nlines ? q : 0));
+    const float2 *X = reinterpret_cast<const float2 *>(src) + (size_t)pr.row * CX + k;
+    const float2 xa = X[0], xb = pr.two ? X[CX] : make_float2(0.f, 0.f);
     float2 *z = A + q * P;
     if (k == 0) {
       z[0] = make_float2(xa.x, xb.x);
@@ -327,15 +345,16 @@ __device__ __forceinline__ void rows_inv_odd(const float *src, float *dst, const
 #pragma unroll 1
   for (int t = tid; t < B * M; t += NTH) {
     const int q = t / M, j = t % M;
-    if (2 * q >= nrows) continue;
-    const bool two = 2 * q + 1 < nrows;
+    if (q >= nlines) continue;
+    const RowPair pr = row_pair(a, line0 + q);
+    const bool two = pr.two;
     const float2 *o = A + q * P + line_slot(l, S, j);
     float2 v[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) v[i] = o[i * ST];
     line_twiddle<R, 1>(l, S, j, v, tw);
     Dft<R, 1>::run(v);
-    const long long e = (row0 + 2 * q) * RX + j;
+    const size_t e = (size_t)pr.row * RX + j;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       v[i] = cscale(v[i], scale);
@@ -355,19 +374,18 @@ __global__ void __launch_bounds__(kRowThreads, kRowMinBlocks) k_row_pass(const _
   using C = RowCfg<NX>;
   extern __shared__ float4 sm4[];
   float2 *A = reinterpret_cast<float2 *>(sm4);
-  constexpr int RPC = C::ODD ? 2 * C::kB : C::kB;  // rows per CTA
-  const long long row0 = (long long)blockIdx.x * RPC;
+  const uint32_t line0 = blockIdx.x * C::kB;
   const int g = blockIdx.y;
-  const int n = (int)(a.nrows - row0 < RPC ? a.nrows - row0 : RPC);
+  const int n = (int)(a.nlines - line0 < C::kB ? a.nlines - line0 : C::kB);
   const float *src = a.g.src[g];
   float *dst = a.g.dst[g];
   const float s = a.g.scale[g];
   if constexpr (C::ODD) {
-    if constexpr (DIR < 0) rows_fwd_odd<NX, kRowThreads>(src, dst, row0, n, s, a.tw, A, threadIdx.x);
-    else rows_inv_odd<NX, kRowThreads>(src, dst, a.g.add[g], row0, n, s, a.tw, A, threadIdx.x);
+    if constexpr (DIR < 0) rows_fwd_odd<NX, kRowThreads>(a, src, dst, line0, n, s, a.tw, A, threadIdx.x);
+    else rows_inv_odd<NX, kRowThreads>(a, src, dst, a.g.add[g], line0, n, s, a.tw, A, threadIdx.x);
   } else {
-    if constexpr (DIR < 0) rows_fwd_even<NX, kRowThreads>(src, dst, row0, n, s, a.tw, a.post, A, threadIdx.x);
-    else rows_inv_even<NX, kRowThreads>(src, dst, a.g.add[g], row0, n, s, a.tw, a.post, A, threadIdx.x);
+    if constexpr (DIR < 0) rows_fwd_even<NX, kRowThreads>(src, dst, line0, n, s, a.tw, a.post, A, threadIdx.x);
+    else rows_inv_even<NX, kRowThreads>(src, dst, a.g.add[g], line0, n, s, a.tw, a.post, A, threadIdx.x);
   }
 }
 
@@ -529,8 +547,7 @@ int launch_rows(const RowPassArgs &a, int ngrids, cudaStream_t s) {
   const size_t sm = C::smem(DIR);
   int rc = func_smem((const void *)k_row_pass<NX, DIR>, sm);
   if (rc) return rc;
-  constexpr int RPC = C::ODD ? 2 * C::kB : C::kB;
-  k_row_pass<NX, DIR><<<dim3((unsigned)((a.nrows + RPC - 1) / RPC), (unsigned)ngrids), kRowThreads, sm, s>>>(a);
+  k_row_pass<NX, DIR><<<dim3((a.nlines + C::kB - 1) / C::kB, (unsigned)ngrids), kRowThreads, sm, s>>>(a);
   CRAVA_LAUNCH_CHECK();
   return CRAVA_GPU_OK;
 }

@@ -139,7 +139,10 @@ int rows_batch(const FftPlans &p, const GridBatch &b, int dir, cudaStream_t s) {
     a.g.add[i] = b.add[i];
     a.g.scale[i] = b.scale[i];
   }
-  a.nrows = (long long)p.g.nyp * p.g.nzp;
+  const int pairs = (p.g.nyp + 1) / 2;
+  a.nlines = (uint32_t)(p.g.nxp % 2 ? pairs : p.g.nyp) * (uint32_t)p.g.nzp;  // sides up to 4096
+  a.odd = (uint32_t)(p.g.nyp % 2);
+  a.fpairs = make_fastdiv((uint32_t)pairs);
   a.tw = dir < 0 ? p.pass.xf : p.pass.xi;
   a.post = p.pass.wx;
   return row_launch(p.g.nxp)(a, b.n, dir, s);

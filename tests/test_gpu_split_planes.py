@@ -1,8 +1,10 @@
-"""256x256 planes, which the fused x + y pass splits over two CTAs: the last y
+"""The x and y passes of slabs, and the planes they work on.
+
+256x256 planes, which the fused x + y pass splits over two CTAs: the last y
 step over the two parts is the z pass's first butterfly where that z pass
 follows, and the plane kernel's own where it does not (the x and y passes of a
 slab, a z pass that the tuning names).  Both are one pass over the plane and
-give the same values."""
+give the same values.  Slab by slab the passes give the whole grid's values."""
 import numpy as np
 import pytest
 import torch
@@ -77,6 +79,7 @@ def test_fused_pass_on_at_any_depth(nz, tile_z):
     ((256, 256, 192), (64, 128)),  # the other way round
     ((128, 128, 54), (24, 30)),
     ((64, 48, 50), (25, 25)),
+    ((25, 27, 50), (25, 25)),      # odd rows, an odd number of them in a slab
 ])
 def test_slabs_equal_the_whole_transform(shape, slabs):
     """The x and y passes slab by slab and the z pass are the 3-D transform of
@@ -99,3 +102,20 @@ def test_slabs_equal_the_whole_transform(shape, slabs):
     for ctx, s in parts:
         ctx.fft_xy(b[s], 1, api.PARAMETER, nz)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("direction", [-1, 1])
+def test_odd_rows_keep_to_their_plane(direction):
+    """Odd rows are transformed two per line: the last row of a plane of an odd
+    number of them is not paired with the next plane's first, so a plane that
+    is not finite leaves the others' values alone, bit for bit."""
+    nx, ny, nz = 25, 27, 24
+    ctx = _context(nx, ny, nz)
+    a = _grid(nx, ny, nz)
+    b = a.clone()
+    b[11] = float("nan")
+    for g in (a, b):
+        ctx.fft_xy(g, direction, api.PARAMETER)
+    assert bool(torch.isnan(b[11][..., :nx]).all())
+    rest = [z for z in range(nz) if z != 11]
+    assert torch.equal(a[rest], b[rest])
