@@ -4,7 +4,7 @@ Each translation unit is compiled with
   nvcc -gencode arch=compute_100a,code=sm_100a -lineinfo -O3
 and linked into one shared library with a static CUDA runtime.  The files
 that must round like the reference's FP32 code (solve_ref.cu, sim.cu) are
-compiled with -fmad=false.
+compiled with -fmad=false.  fft_len.cu is compiled once per line length.
 """
 from __future__ import annotations
 
@@ -26,14 +26,6 @@ SOURCES = {
     "cols_tma.cu": [],
     "pass.cu": [],
     "plane.cu": [],
-    "fft_len0.cu": [],
-    "fft_len1.cu": [],
-    "fft_len2.cu": [],
-    "fft_len3.cu": [],
-    "fft_len4.cu": [],
-    "fft_len5.cu": [],
-    "fft_len6.cu": [],
-    "fft_len7.cu": [],
     "solve.cu": [],
     "solve_ref.cu": ["-fmad=false"],
     "sim.cu": ["-fmad=false"],
@@ -48,6 +40,17 @@ SOURCES = {
     "divide.cu": [],
     "interp.cu": [],
 }
+
+
+def _smooth(n):
+    for p in (2, 3, 5, 7):
+        while n % p == 0:
+            n //= p
+    return n == 1
+
+
+# csrc/fft_lengths.cuh lists the same
+LENGTHS = [n for n in range(24, 513) if _smooth(n)]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
          "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
@@ -60,15 +63,21 @@ def _newer(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def units():
+    """(source, object, flags) of every translation unit."""
+    return ([(src, src.replace(".cu", ".o"), flags) for src, flags in SOURCES.items()]
+            + [("fft_len.cu", f"fft_len{n}.o", [f"-DCRAVA_LENGTH={n}"]) for n in LENGTHS])
+
+
 def build(verbose: bool = False, force: bool = False, extra=()) -> str:
     os.makedirs(OBJ, exist_ok=True)
     os.makedirs(os.path.dirname(LIB), exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     headers.append(os.path.join(ROOT, "include", "crava_gpu.h"))
     objs, cmds = [], []
-    for src, flags in SOURCES.items():
+    for src, obj, flags in units():
         s = os.path.join(CSRC, src)
-        o = os.path.join(OBJ, src.replace(".cu", ".o"))
+        o = os.path.join(OBJ, obj)
         objs.append(o)
         if force or _newer(o, [s] + headers):
             cmds.append([NVCC, *ARCH, *FLAGS, *flags, *extra, "-c", s, "-o", o])

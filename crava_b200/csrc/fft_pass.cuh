@@ -566,7 +566,7 @@ int launch_cols(const ColPassArgs &a, int ngrids, cudaStream_t s) {
 // The z pass that completes the y transform of planes split in two (plane.cu).
 int z_parts_launch(const ColPassArgs &a, int n, int ngrids, int dir, cudaStream_t s);
 
-// The compiled lengths, each in one of the files fft_len<k>.cu.
+// The compiled lengths (fft_len.cu).
 using ColLaunch = int (*)(const ColPassArgs &, int ngrids, int dir, cudaStream_t);
 using RowLaunch = int (*)(const RowPassArgs &, int ngrids, int dir, cudaStream_t);
 ColLaunch col_launch(int n);  // null: not compiled
@@ -579,20 +579,17 @@ template <int NX>
 int run_rows(const RowPassArgs &a, int ngrids, int dir, cudaStream_t s) {
   return dir < 0 ? launch_rows<NX, -1>(a, ngrids, s) : launch_rows<NX, 1>(a, ngrids, s);
 }
-#define CRAVA_COL_CASE(N) case N: return run_cols<N>;
-#define CRAVA_ROW_CASE(N) case N: return run_rows<N>;
-#define CRAVA_SYNT_CASE(N) case N: return synt_list(N).n < 2 ? nullptr : run_synt_pass<N>;
-#define CRAVA_LENGTHS(K)                                                    \
-  namespace crava {                                                         \
-  ColLaunch col_launch_##K(int n) {                                         \
-    switch (n) { CRAVA_COLS(CRAVA_COL_CASE) default: return nullptr; }      \
-  }                                                                         \
-  RowLaunch row_launch_##K(int nx) {                                        \
-    switch (nx) { CRAVA_ROWS(CRAVA_ROW_CASE) default: return nullptr; }     \
-  }                                                                         \
-  SyntLaunch synt_launch_##K(int n) {                                       \
-    switch (n) { CRAVA_COLS(CRAVA_SYNT_CASE) default: return nullptr; }     \
-  }                                                                         \
-  }
+// Rows: the even ones 32 .. 512 and the odd ones 25 .. 255.
+template <int NX>
+RowLaunch row_of() {
+  if constexpr (NX % 2 == 0 ? NX >= 32 : NX <= 255) return run_rows<NX>;
+  else return nullptr;
+}
+// Synthetic seismic: the lengths of two or three stages of its radices.
+template <int N>
+SyntLaunch synt_of() {
+  if constexpr (synt_list(N).n >= 2) return run_synt_pass<N>;
+  else return nullptr;
+}
 
 }  // namespace crava

@@ -4,41 +4,35 @@
 
 #include <vector>
 
+#include "fft_lengths.cuh"
 #include "fft_pass.cuh"
 
 namespace crava {
 
-#define CRAVA_EIGHTHS(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
-#define CRAVA_DECL(K)           \
-  ColLaunch col_launch_##K(int); \
-  RowLaunch row_launch_##K(int); \
-  SyntLaunch synt_launch_##K(int);
-CRAVA_EIGHTHS(CRAVA_DECL)
+#define CRAVA_DECL(N)        \
+  ColLaunch col_launch_##N(); \
+  RowLaunch row_launch_##N(); \
+  SyntLaunch synt_launch_##N();
+CRAVA_LINE_LENGTHS(CRAVA_DECL)
 #undef CRAVA_DECL
 
+#define CRAVA_FIND(N) case N: return CRAVA_WHICH(N)();
+#define CRAVA_WHICH(N) col_launch_##N
 ColLaunch col_launch(int n) {
-#define CRAVA_FIND(K) \
-  if (ColLaunch f = col_launch_##K(n)) return f;
-  CRAVA_EIGHTHS(CRAVA_FIND)
-#undef CRAVA_FIND
-  return nullptr;
+  switch (n) { CRAVA_LINE_LENGTHS(CRAVA_FIND) default: return nullptr; }
 }
-
+#undef CRAVA_WHICH
+#define CRAVA_WHICH(N) row_launch_##N
 RowLaunch row_launch(int nx) {
-#define CRAVA_FIND(K) \
-  if (RowLaunch f = row_launch_##K(nx)) return f;
-  CRAVA_EIGHTHS(CRAVA_FIND)
-#undef CRAVA_FIND
-  return nullptr;
+  switch (nx) { CRAVA_LINE_LENGTHS(CRAVA_FIND) default: return nullptr; }
 }
-
+#undef CRAVA_WHICH
+#define CRAVA_WHICH(N) synt_launch_##N
 SyntLaunch synt_launch(int n) {
-#define CRAVA_FIND(K) \
-  if (SyntLaunch f = synt_launch_##K(n)) return f;
-  CRAVA_EIGHTHS(CRAVA_FIND)
-#undef CRAVA_FIND
-  return nullptr;
+  switch (n) { CRAVA_LINE_LENGTHS(CRAVA_FIND) default: return nullptr; }
 }
+#undef CRAVA_WHICH
+#undef CRAVA_FIND
 
 namespace {
 

@@ -298,13 +298,9 @@ int launch_synt_pass(const SyntPassArgs &a, cudaStream_t s) {
 }
 template <int N>
 int run_synt_pass(const SyntPassArgs &a, cudaStream_t s) {
-  if constexpr (synt_list(N).n < 2) {
-    return CRAVA_GPU_ERR_ARG;
-  } else {
-    return SyntCfg<N, 8>::smem(a.nt) <= 220 * 1024 ? launch_synt_pass<N, 8>(a, s) : launch_synt_pass<N, 4>(a, s);
-  }
+  return SyntCfg<N, 8>::smem(a.nt) <= 220 * 1024 ? launch_synt_pass<N, 8>(a, s) : launch_synt_pass<N, 4>(a, s);
 }
-// The compiled lengths (fft_len<k>.cu); null: none.
+// The compiled lengths (fft_len.cu); null: none.
 using SyntLaunch = int (*)(const SyntPassArgs &, cudaStream_t);
 SyntLaunch synt_launch(int n);
 
