@@ -42,7 +42,15 @@ struct RowPassArgs {
   const float2 *post; // W_nxp^k, k <= nxp / 2 (even nxp)
 };
 
-constexpr int kRowThreads = 256, kRowMinBlocks = 4;
+// Small CTAs, about 1024 points on 128 threads and eight resident per SM: one's
+// barriers then wait for few warps while the others load and store.  256 threads
+// with 4096 points and four per SM took longer in every pass that is not launch
+// bound, and longer than the register-resident pass of fft.cu at 64 and 256
+// points inverse: us forward / inverse, 128 x 64 x 64 rows 8.6 / 8.6 -> 6.6 / 6.8,
+// 512 x 256 x 256 54 / 66 -> 52 / 62, 96 x 200 x 300 18.7 / 16.7 -> 15.2 / 14.7, 200 x
+// 200 x 192 22.9 / 20.9 -> 22.8 / 18.8; with 2048 points 7.6 / 8.5 at the first, 16.9 /
+// 14.7 at the third and the same at the others.
+constexpr int kRowThreads = 128, kRowMinBlocks = 8;
 
 template <int NX>
 struct RowCfg {
@@ -54,8 +62,8 @@ struct RowCfg {
   using I = LineOf<N, kBanks.si, true>;   // inverse: last radix small (long runs of stores)
   static constexpr int PF = kBanks.pf, PI = kBanks.pi;
   static_assert(PF >= F::R(0) * F::S(0) && PI >= I::R(0) * I::S(0), "a row holds its line");
-  // lines per CTA: about 4096 points
-  static constexpr int kB = 4096 / N < 8 ? 8 : 4096 / N > 64 ? 64 : 4096 / N / 8 * 8;
+  // lines per CTA: about 1024 points
+  static constexpr int kB = 1024 / N < 8 ? 8 : 1024 / N > 32 ? 32 : 1024 / N / 8 * 8;
   static constexpr int NP = N / 2 + N % 2;  // position pairs of an even row
   static constexpr size_t smem(int dir) { return sizeof(float2) * (size_t)kB * (dir < 0 ? PF : PI); }
 };
