@@ -430,9 +430,19 @@ struct ColCfg {
     for (int s = 0; s < L::nst(); ++s) m = L::R(s) > m ? L::R(s) : m;
     return m;
   }
+  static constexpr int min_m() {
+    int m = N;
+    for (int s = 0; s < L::nst(); ++s) m = L::M(s) < m ? L::M(s) : m;
+    return m;
+  }
   // butterflies of a line that run at once: those of a stage in one round
-  // where at most 20, else in equal rounds
-  static constexpr int kRounds = ceil_div(max_m(), 20);
+  // where at most 20, else in equal rounds.  Where one stage has half of the
+  // other's (128 = 16 x 8, 162, 200 = 20 x 10) the smaller number, so that no
+  // thread idles in that stage: a unit of 256x128x128, three angles, 486 -> 466 us
+  // (480 with the register-resident passes), of 96x200x300 727 -> 709.  Two rounds
+  // where the stages are alike cost instead: 128x256x256 931 -> 1139.
+  static constexpr bool kHalf = min_m() >= 8 && max_m() <= 20 && max_m() == 2 * min_m();
+  static constexpr int kRounds = kHalf ? 2 : ceil_div(max_m(), 20);
   static constexpr int TPB = (ceil_div(max_m(), kRounds) + 1) / 2 * 2;
   static constexpr int NTH = kColLines * TPB;
   static constexpr int kHold = 16;  // points a thread's loads in flight cover (at least a radix)
