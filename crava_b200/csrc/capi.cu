@@ -156,17 +156,25 @@ void prof_collect(crava_gpu_ctx *c) {
 
 // How n transforms of the built-in passes are spread: grids per launch, and
 // transform lanes (of the context's) they run on.
+// Measured as units, us, in 23 sizes of 2 to 126 MB per grid against other lines
+// (12, 36, 48 MB per launch; 75, 140 MB of L2; all lanes; one launch):
 //  * A pass over small grids is shorter than a launch, so they share one: all
-//    of them up to 48 MB together, else 24 MB at a time (13 grids of 64x64x128:
-//    92 us per unit in one launch, 96 us in 24 MB launches).
+//    of them up to 48 MB together (13 grids of 64x64x128, 2 MB: 90, in 24 MB
+//    launches 94; with up to 100 MB together 100x100x200, 8 MB, takes 305, not
+//    296, and nothing gains), else 24 MB at a time (12 MB: 96x96x128, 5 MB, 211 for
+//    175; 36 or 48 MB: 160x160x160, 17 MB, 553 for 517, though 96x96x128 would
+//    take 165).
 //  * A grid that with those in flight on the other lanes fits the L2 (126 MB)
-//    goes through its passes there: as many lanes as fit 100 MB (96x200x300, 24
-//    MB: 0.88 ms per unit on 3 lanes against 1.02 ms in one launch per pass;
-//    192x160x384, 48 MB: 1.86 ms on 2 lanes, 1.99 on 3, 1.96 in one launch).
+//    goes through its passes there: as many lanes as fit 100 MB (five angles:
+//    96x200x300, 24 MB, 835 on 3 lanes, 910 in one launch per pass; 128x256x256,
+//    34 MB, 1087 on 2, 1140 on 3; 192x160x384, 48 MB, 1706 on 2, 1813 on 3, 1749 on
+//    one.  160x160x320, 33 MB, would rather have one launch: 1163 for 1223).
 //  * Larger grids stream from HBM whatever the order: one launch per pass for
-//    all of them has no tails between grids (256x256x512: 4.90 ms per unit
-//    against 5.03 ms on 3 lanes, both before the plane passes' fetch into L2,
-//    which also looks ahead from grid to grid of a launch: 4.47).
+//    all of them has no tails between grids, and the plane passes' fetch into L2
+//    looks ahead from grid to grid (three angles: 224x224x320, 65 MB, 2017, on 3
+//    lanes 2046; 256x256x256, 68 MB, 1865 and 1957; 240x256x400, 99 MB, 3044 and
+//    3128; 250x250x500, 126 MB, 4594 and 4763; at 240x240x240, 56 MB, two lanes
+//    would take 1703 for 1737).
 constexpr double kOneLaunch = 48e6, kPerLaunch = 24e6, kInL2 = 100e6;
 struct Spread {
   int per, lanes;

@@ -39,8 +39,9 @@ using namespace crava;
 
 namespace {
 
-// 255 registers: two blocks of 128 threads per SM, so that the planes' shares
-// end within a block's length of each other
+// Blocks of 128 threads, so that the planes' shares end within a block's length
+// of each other: two per SM from four angles on (216 and 255 registers), three at
+// two and three angles, seven at one
 constexpr int kThreads = 128;
 using sb::tri;
 
@@ -348,8 +349,8 @@ extern "C" int crava_gpu_loglik_grad(crava_gpu_ctx *c, const crava_gpu_grids *gr
   a.cnxp = c->g.cnxp; a.nxp = c->g.nxp;
   a.plane = (long long)c->g.cnxp * c->g.nyp;
   // Blocks over the inverted planes alone, about four bins per thread where
-  // the grid has enough of them for eight rounds of the device's resident
-  // blocks, else fewer: the last round's idle share stays small
+  // the grid has enough of them for eight rounds of 296 resident blocks (two per
+  // SM), else fewer: the last round's idle share stays small
   // (192x160x384x5: 625 us with two 256-thread blocks for every plane of the
   // grid, two rounds of which the second was nearly empty).
   a.planes = c->tables.n_inv > 0 ? c->tables.order_inv : nullptr;

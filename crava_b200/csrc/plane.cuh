@@ -3,8 +3,9 @@
 // shared memory between the two passes, so a transform moves 4 grids of HBM
 // traffic (this pass and the z pass) where separate x, y and z passes move 6.
 //
-// Planes up to 128x128 are one CTA's (CS = 1; 75 KB, three CTAs per SM).  Of a
-// 256x256 plane CTA r of CS = 2 holds the rows y = CS q + r, q < NQ = nyp / CS
+// Planes up to 128x128, and 256x64, are one CTA's (CS = 1): 23 to 45 KB and 256
+// threads up to 64x128 and 128x64, 88 and 78 KB, 512 threads and two CTAs per SM at
+// 128x128 and 256x64.  Of a 256x256 plane CTA r of CS = 2 holds the rows y = CS q + r, q < NQ = nyp / CS
 // (149 KB, 1024 threads).  With ky = k1 + NQ k2,
 //   Y[k1 + NQ k2] = sum_r W_CS^{r k2} [ W_nyp^{r k1} sum_q x[CS q + r] W_NQ^{q k1} ]:
 // the kernel does the brackets, leaves bracket (k1, r) in row k1 + NQ r, and the

@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThreads) k_noise_filter(NoiseFilterArgs a) {
 // stream's once per block, and eight rounds are left per value, the last two of
 // them only as far as the two words that are used depend on them.  Same words
 // as philox10.  The filter is bound by instruction issue (8 realisations of
-// 256 x 256 x 512: 3.7 GB, 0.56 ms at copy rate): 2.61 ms with ten whole rounds
+// 256 x 256 x 512: 4.06 GB, 0.62 ms at copy rate): 2.61 ms with ten whole rounds
 // per value, 2.19 ms so.
 struct BinPart {
   uint32_t a, b, w;
