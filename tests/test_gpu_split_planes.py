@@ -119,3 +119,25 @@ def test_odd_rows_keep_to_their_plane(direction):
     assert bool(torch.isnan(b[11][..., :nx]).all())
     rest = [z for z in range(nz) if z != 11]
     assert torch.equal(a[rest], b[rest])
+
+
+def test_whole_planes_of_several_grids_in_one_launch():
+    """Realisations with their means through the pass that completes y, three
+    grids per launch, against the separate passes (float32 rounding of one
+    inverse transform each, and of the mean's addition)."""
+    nx, ny, nz = 256, 256, 24
+    ctx = _context(nx, ny, nz)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    full = (nz, ny, 2 * (nx // 2 + 1))
+    cov = [torch.zeros(full, device="cuda") for _ in range(6)]
+    for c in cov[:3]:
+        c[..., 0::2] = 0.5 + torch.rand(full[:2] + (full[2] // 2,), device="cuda", generator=gen)
+    mean = [torch.randn(full, device="cuda", generator=gen) for _ in range(3)]
+    outs = {}
+    for xy in (1, 0):
+        ctx.set_tuning(-1, -1, 0, 3, -1, None, xy)
+        outs[xy] = [torch.empty(full, device="cuda") for _ in range(12)]
+        ctx.simulate(cov, mean, 5, 0, outs[xy])
+    for a, b in zip(outs[1], outs[0]):
+        a, b = a[..., :nx].double(), b[..., :nx].double()
+        assert float((a - b).norm() / b.norm()) < 2 * 7.6e-7
