@@ -293,9 +293,10 @@ int crava_gpu_posterior_noalloc(const crava_gpu_params *params,
  * bit for bit, the built-in ones agree with them to float rounding.  xy_fused:
  * the x and y passes as one kernel where the plane has one (sides 64 and
  * 128, 256x64, 256x256; 0 off, 1 on, -1 built-in = on there unless the tuning
- * names another x or y pass, at 256x256 for nzp 64, 128, 256 and 512); it factorises the y transform differently, so it agrees with the
- * separate passes to float rounding, not bit for bit.  kappa_refine (mixed form only, >= 0): an inverted bin whose
- * FP32 factor has (max L_ii / min L_ii)^2 above it takes one FP64
+ * names another x or y pass, at 256x256 for nzp 64, 128, 256 and 512); it
+ * factorises the y transform differently, so it agrees with the separate
+ * passes to float rounding, not bit for bit.  kappa_refine (mixed form only,
+ * >= 0): an inverted bin whose FP32 factor has (max L_ii / min L_ii)^2 above it takes one FP64
  * refinement step (0 refines every bin).  solve_shape: the launch shape of
  * the FP64 and mixed solves (-1 built-in: the Woodbury kernel (shape 6)
  * for FP64 on a context, the register-factor kernel with four 128-thread
